@@ -4,8 +4,9 @@
 A case is a dict of plain values:
 
   kind      "run"     sl_run: MCMC of `chains` replicate chains, scored every
-                      `period` iterations; with `batch` pedigrees of uneven
-                      sizes, one sl_batch_run with MC3 exchanges
+                      `period` iterations (0: burn-in, nothing scored); with
+                      `batch` pedigrees of uneven sizes, one sl_batch_run with
+                      MC3 exchanges
             "impute"  sl_sequential_imputation_run: legal starting graphs
             "score"   sl_lod_score_graphs: stored graphs scored
             "adjoint" sl_trait_backward: gradients of the trait peel
@@ -50,12 +51,12 @@ def listed():
         dict(small, **dict(fast, precision="exact"), name="run exact 30x200 c2", chains=2, iterations=4, period=2),
         # the program's ordinary run: a large family, replicate chains, L- and M-sweeps mixed, graphs scored
         dict(mid, **fast, name="run 120x2000 c10", chains=10, iterations=10, period=5),
-        # its two sweeps apart: locus sampler only, meiosis sampler only
-        dict(mid, **dict(fast, lprob=1.0), name="lsweep 120x2000 c10", chains=10, iterations=8, period=8),
-        dict(mid, **dict(fast, lprob=0.0), name="msweep 120x2000 c10", chains=10, iterations=4, period=4),
-        # the largest pedigree that the configurations hold, dense map
-        dict(large, **dict(fast, lprob=1.0), name="lsweep 400x10000 c8", chains=8, iterations=4, period=4),
-        dict(large, **dict(fast, lprob=0.0), name="msweep 400x10000 c8", chains=8, iterations=1, period=1),
+        # burn-in with its two sweeps apart: locus sampler only, meiosis sampler only
+        dict(mid, **dict(fast, lprob=1.0), name="lsweep 120x2000 c10", chains=10, iterations=8, period=0),
+        dict(mid, **dict(fast, lprob=0.0), name="msweep 120x2000 c10", chains=10, iterations=4, period=0),
+        # the same on the largest pedigree that the configurations hold, dense map
+        dict(large, **dict(fast, lprob=1.0), name="lsweep 400x10000 c8", chains=8, iterations=4, period=0),
+        dict(large, **dict(fast, lprob=0.0), name="msweep 400x10000 c8", chains=8, iterations=2, period=0),
         # a batch of uneven pedigrees, some founders untyped, MC3 chains with exchanges, odd marker count
         dict(small, **fast, name="batch mc3 6x301 c8", members=100, generations=5, loops=2, affected=10, pedigree=11,
              markers=301, untyped=0.2) | dict(batch=6, chains=8, iterations=10, period=5),
@@ -83,11 +84,13 @@ def draw(rng):
     if kind == "run":
         exact = n <= 60 and rng.random() < 0.25
         c |= dict(precision="exact" if exact else "fast", batch=1, lprob=rng.choice([0.0, 0.5, 1.0]),
-                  chains=log(1, 3 if exact else 12), iterations=2 if exact else 4, period=2)
+                  chains=log(1, 3 if exact else 12), iterations=2 if exact else 4)
+        # pedigrees whose compiled scorer takes long to build: burn-in
+        c["period"] = 0 if n > 130 else rng.choice([0, 2])
         if exact:
             c["markers"] = min(c["markers"], 300)
         elif n <= 100 and rng.random() < 0.3:
-            c |= dict(batch=rng.randint(2, 5), markers=min(c["markers"], 500), lprob=0.5, chains=rng.randint(2, 8))
+            c |= dict(batch=rng.randint(2, 5), markers=min(c["markers"], 500), lprob=0.5, chains=rng.randint(2, 8), period=2)
     elif kind == "impute":
         c |= dict(precision="fast", markers=log(60, 400), chains=rng.randint(1, 6), passes=log(8, 250))
     elif kind == "score":
@@ -202,10 +205,9 @@ def prepare(case, seed):
         elif case.get("lod") == "fp64" or case["kind"] == "adjoint":
             opt |= dict(sampler_precision=api.SL_SAMPLER_FAST, lod_precision=api.SL_LOD_FP64)
         else:
-            # the program's choice of scorer: the form compiled for the pedigree; samplers alone and the largest
-            # pedigrees, whose compile takes long, score with the interpreter
-            jit = case["kind"] == "score" or (case["kind"] == "run" and case["lprob"] == 0.5 and fam["N"] <= 150
-                                              and len(fams) == 1)
+            # the program's choice of scorer: the form compiled for the pedigree; the batch's pedigrees are scored
+            # by the interpreter, and nothing is compiled where nothing is scored
+            jit = case["kind"] == "score" or (case["kind"] == "run" and case["period"] > 0 and len(fams) == 1)
             opt |= dict(sampler_precision=api.SL_SAMPLER_FAST, lod_precision=api.SL_LOD_FP32_RESCALED,
                         lod_kernel=api.SL_LOD_KERNEL_JIT_REG if jit else api.SL_LOD_KERNEL_INTERP)
         ctx = api.Context(prob, **opt)
@@ -233,14 +235,17 @@ def run(s):
         for ctx, dg in zip(s["ctx"], s["dg"]):
             ctx.set_graphs(dg)
             ctx.lod_reset()
-        o = dict(iterations=case["iterations"], period=case["period"], lprob=case["lprob"], seed=s["seed"])
+        o = dict(lprob=case["lprob"], seed=s["seed"])
+        o |= (dict(iterations=case["iterations"], period=case["period"]) if case["period"]
+              else dict(iterations=0, burnin=case["iterations"]))
         if "batch" in s:
             s["batch"].run(exchange_period=case["period"], **o)
         else:
             s["ctx"][0].run(**o)
         for k, (ctx, g) in enumerate(zip(s["ctx"], s["out"])):
-            raw, count, tp = ctx.lod_results()
-            out["lod%d" % k], out["count%d" % k], out["trait%d" % k] = raw, int(count), tp
+            if case["period"]:
+                raw, count, tp = ctx.lod_results()
+                out["lod%d" % k], out["count%d" % k], out["trait%d" % k] = raw, int(count), tp
             out["graphs%d" % k] = ctx.get_graphs(out=g)
     elif case["kind"] == "impute":
         ctx = s["ctx"][0]
@@ -272,7 +277,7 @@ def work(case):
         cells = sum(4.0 ** (len(c) + 1) for c in fam["op_cutset"])   # a trait peel's terms over every state
         if case["kind"] == "run":
             C, it = case["chains"], case["iterations"]
-            scored = C * (-(-it // case["period"]))
+            scored = C * (-(-it // case["period"])) if case["period"] else 0
             b += C * (2 * graph + it * step_bytes(N, F, M)) + scored * npos * position_bytes(N, F, N_LOD)
             # an L-sweep: two passes over the peel, about two allowed cells of two states each, four factors a term
             l_sweep = 2.0 * M * K * 2 * 2 * 4
