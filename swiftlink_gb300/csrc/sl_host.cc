@@ -41,7 +41,8 @@ cudaError_t launch_msampler(const ProblemDev& P, uint32_t* dg, int first, int nc
                             int64_t mstride, int nm, const double* u, int64_t ucs, uint64_t seed, uint64_t iter,
                             const uint8_t* sel, int want, double* raw64, float* raw32, void* fb, uint8_t* badc,
                             uint8_t* maps, int* status, int fag_threads, int exact, cudaStream_t s,
-                            const uint64_t* key = nullptr, double* ubuf = nullptr, int pairs = 0);
+                            const uint64_t* key = nullptr, double* ubuf = nullptr, int chains = 1, int load = 1);
+int64_t msweep_launches(const ProblemDev& P, int chains, int nm);
 cudaError_t launch_set_key(uint64_t* key, uint64_t seed, uint64_t iter, cudaStream_t s);
 cudaError_t launch_lfreq(const double* minor, float2* out, int64_t n, cudaStream_t s);
 cudaError_t launch_si(const ProblemDev& P, uint32_t* dg, int first, int nchain, const int32_t* starts,
@@ -98,6 +99,7 @@ struct sl_ctx {
     cudaStream_t lstream = nullptr;   // L-sweeps of device-driven runs, concurrent with M-sweeps
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     int n_chains = 0;
+    int sweep_load = 1;              // chains whose sweeps may run at once: the context's, or its batch's while that is captured
     int lod_precision = 0;
     int sampler_precision = 0;
     int sms = 0;
@@ -239,14 +241,13 @@ cudaEvent_t take_event(sl_ctx* c) {
     return e;
 }
 // Bracket one launch with events when profiling is on.
-// Kernels one M-sweep of nm meioses launches for a chain: a reset, then per
-// meiosis a likelihood and a filter kernel.
-static int64_t msweep_kernels(const sl_ctx*, int nm) { return 1 + 2 * (int64_t)nm; }
-
-// The fast M-step's likelihood kernel puts two loci in a warp (fewer
-// instructions per locus, a longer launch) when the context holds enough
-// chains for the GPU to be throughput-bound.
-static int msampler_pairs(const sl_ctx* ctx) { return ctx->n_chains >= 8 ? 1 : 0; }
+// Kernels one M-sweep of nm meioses launches for a chain: in the fast mode one
+// (a cluster per chain), else a reset, then per meiosis a likelihood and a
+// filter kernel.
+static int64_t msweep_kernels(const sl_ctx* ctx, int nm) {
+    if (ctx->sampler_precision == SL_SAMPLER_EXACT) return 1 + 2 * (int64_t)nm;
+    return msweep_launches(ctx->P, ctx->n_chains, nm);
+}
 
 // An L-sampler launch: the kernel specialised to the pedigree when it was
 // built, else the generic one.
@@ -690,6 +691,141 @@ static void pack_graphs(const int32_t* src, int n, int N, int F, int M, int W, u
 static void unpack_graphs(const uint32_t* src, int n, int N, int F, int M, int W, int32_t* dst) {
     for_columns((size_t)n * M, (size_t)n * M * N * 8,
                 [&](size_t a, size_t b) { unpack_columns(src, N, F, W, dst, a, b); });
+}
+
+// What a locus's genotypes alone say about toggling a meiosis there
+// (ProblemDev::mflip; the M-sweep evaluates the founder-allele graph only
+// where neither mask holds).  Toggling meiosis (i, p) -- the allele that i has
+// from its parent p -- moves it, and what i's descendants have of it, from one
+// founder allele a of p's two to the other, b; nobody else's alleles change.
+//   same:  nobody at or below i is typed, so the graph has the same edges; or
+//          a and b are both fixed, to one colour, by homozygous members that
+//          the toggle does not move (p itself, or, where p is untyped, both of
+//          p's parents), so every edge that moves from a to b meets the same
+//          colour, at the same point of the evaluation: the same terms.
+//   never: the members outside i's descendants fix a and b to opposite colours
+//          (p is heterozygous and they fix one of them, or p is untyped between
+//          two unlike homozygous parents), and i's genotype, with its other
+//          parent's alleles fixed by them too where i is heterozygous, tells
+//          the moving allele's colour: it cannot be both a's and b's.
+// Both hold when the graph as it is is legal; the sweep evaluates the rest.
+// planes: [N][words] bits over the loci.
+static std::vector<uint32_t> meiosis_flips(const sl_problem_desc* d, const std::vector<uint8_t>& geno, int words) {
+    const int N = d->n_members, F = d->n_founders, M = d->n_markers;
+    const size_t W = words;
+    std::vector<uint32_t> hom_a(N * W, 0), hom_b(N * W, 0), het(N * W, 0), below(N * W, 0);
+    {
+        std::vector<uint32_t> a(N), b(N), h(N);   // a word of every member's planes at a time
+        for (int l0 = 0; l0 < M; l0 += 32) {
+            std::fill(a.begin(), a.end(), 0u);
+            std::fill(b.begin(), b.end(), 0u);
+            std::fill(h.begin(), h.end(), 0u);
+            for (int l = l0; l < std::min(M, l0 + 32); ++l) {
+                const uint8_t* row = geno.data() + (size_t)l * N;
+                for (int i = 0; i < N; ++i) {
+                    const uint32_t g = row[i] & 3u;
+                    a[i] |= (uint32_t)(g == G_HOMOZ_A) << (l - l0);
+                    b[i] |= (uint32_t)(g == G_HOMOZ_B) << (l - l0);
+                    h[i] |= (uint32_t)(g == G_HETERO) << (l - l0);
+                }
+            }
+            for (int i = 0; i < N; ++i) {
+                const size_t at = i * W + (l0 >> 5);
+                hom_a[at] = a[i];
+                hom_b[at] = b[i];
+                het[at] = h[i];
+                below[at] = a[i] | b[i] | h[i];   // i typed; its descendants are added next
+            }
+        }
+    }
+    std::vector<std::vector<int>> kids(N);
+    for (int i = F; i < N; ++i) {
+        kids[d->mother[i]].push_back(i);
+        if (d->father[i] != d->mother[i]) kids[d->father[i]].push_back(i);
+    }
+    // a child's children before the child: members at or below each one that are typed
+    std::vector<int> state(N, 0);
+    std::vector<int> stack;
+    for (int r = 0; r < N; ++r) {
+        if (state[r]) continue;
+        stack.push_back(r);
+        while (!stack.empty()) {
+            const int i = stack.back();
+            if (state[i] == 0) {
+                state[i] = 1;
+                for (int k : kids[i])
+                    if (!state[k]) stack.push_back(k);
+                continue;
+            }
+            stack.pop_back();
+            if (state[i] == 2) continue;
+            state[i] = 2;
+            for (int k : kids[i])
+                for (size_t w = 0; w < W; ++w) below[i * W + w] |= below[k * W + w];
+        }
+    }
+    std::vector<uint32_t> out((size_t)2 * (N - F) * 2 * W, 0);
+    std::vector<char> under(N);   // i and its descendants
+    auto hom = [&](int x, size_t w) { return hom_a[x * W + w] | hom_b[x * W + w]; };
+    auto side_of = [&](int parent, int child) { return d->mother[child] == parent ? 0 : 1; };
+    auto other = [&](int child, int side) { return side == 0 ? d->father[child] : d->mother[child]; };
+    auto selfed = [&](int x) { return x >= F && d->mother[x] == d->father[x]; };
+    // Loci where the colours of a heterozygous x's alleles are fixed (one is, so the other is) by members
+    // outside `under`: a homozygous parent, or a child told apart by its own genotype and its other parent's;
+    // one level deeper, by a parent's or another child's alleles that are fixed so.
+    auto fixed1 = [&](int x, size_t w) {
+        uint32_t m = 0;
+        if (x >= F && !selfed(x)) m = hom(d->mother[x], w) | hom(d->father[x], w);
+        for (int k : kids[x])
+            if (!under[k] && !selfed(k)) m |= hom(k, w) | (het[k * W + w] & hom(other(k, side_of(x, k)), w));
+        return m;
+    };
+    auto known = [&](int x, size_t w) {   // both alleles of x are fixed
+        const uint32_t h = het[x * W + w];
+        return hom(x, w) | (h ? h & fixed1(x, w) : 0u);
+    };
+    auto fixed2 = [&](int x, size_t w) {
+        uint32_t m = fixed1(x, w);
+        if (!~m) return m;
+        if (x >= F && !selfed(x)) m |= known(d->mother[x], w) | known(d->father[x], w);
+        for (int k : kids[x])
+            if (!under[k] && !selfed(k) && het[k * W + w]) m |= het[k * W + w] & known(other(k, side_of(x, k)), w);
+        return m;
+    };
+    for (int i = F; i < N; ++i) {
+        std::fill(under.begin(), under.end(), 0);
+        under[i] = 1;
+        stack.assign(1, i);
+        while (!stack.empty()) {
+            const int x = stack.back();
+            stack.pop_back();
+            for (int k : kids[x])
+                if (!under[k]) {
+                    under[k] = 1;
+                    stack.push_back(k);
+                }
+        }
+        for (int side = 0; side < 2; ++side) {
+            uint32_t* same = out.data() + (size_t)(2 * (i - F) + side) * 2 * W;
+            uint32_t* never = same + W;
+            const int p = side == 0 ? d->mother[i] : d->father[i], o = other(i, side);
+            for (size_t w = 0; w < W; ++w) {
+                const uint32_t none = ~(hom(p, w) | het[p * W + w]);   // p untyped
+                uint32_t like = 0, unlike = 0;
+                if (p >= F && !selfed(p)) {
+                    const size_t q0 = d->mother[p] * W + w, q1 = d->father[p] * W + w;
+                    like = (hom_a[q0] & hom_a[q1]) | (hom_b[q0] & hom_b[q1]);
+                    unlike = (hom_a[q0] & hom_b[q1]) | (hom_b[q0] & hom_a[q1]);
+                }
+                same[w] = hom(p, w) | (none & like) | ~below[i * W + w];
+                if (selfed(i) || !~same[w]) continue;
+                const uint32_t apart = (het[p * W + w] & fixed2(p, w)) | (none & unlike);
+                if (apart & ~same[w])
+                    never[w] = apart & ~same[w] & (hom(i, w) | (het[i * W + w] & known(o, w)));
+            }
+        }
+    }
+    return out;
 }
 
 // Peel-operation descriptors with gather maps: for every previous rfunction,
@@ -1279,7 +1415,7 @@ int sl_create(const sl_problem_desc* d, const sl_options* opt, sl_ctx** out) {
 
     ctx = new sl_ctx();
     ctx->device = opt->device;
-    ctx->n_chains = opt->n_chains;
+    ctx->n_chains = ctx->sweep_load = opt->n_chains;
     ctx->lod_precision = opt->lod_precision;
     ctx->sampler_precision = opt->sampler_precision;
     int rc = SL_OK;
@@ -1446,6 +1582,12 @@ int sl_create(const sl_problem_desc* d, const sl_options* opt, sl_ctx** out) {
         if ((rc = upload(ctx, (uint16_t**)&P.typ_ent, ent.data(), ent.size()))) return bail(rc);
         if ((rc = upload(ctx, (uint16_t**)&P.typ_cnt, cnt.data(), cnt.size()))) return bail(rc);
         if ((rc = upload(ctx, (uint16_t**)&P.typ_nhet, nhet.data(), nhet.size()))) return bail(rc);
+    }
+    P.mflip = nullptr;
+    P.mflip_words = (M + 31) / 32;
+    if (P.ls_fast) {
+        const std::vector<uint32_t> mf = meiosis_flips(d, geno, P.mflip_words);
+        if ((rc = upload(ctx, (uint32_t**)&P.mflip, mf.data(), mf.size()))) return bail(rc);
     }
     if ((rc = upload(ctx, (uint8_t**)&P.typed, typed.data(), N))) return bail(rc);
     if ((rc = upload(ctx, (double**)&P.prior, ctx->prior_table.data(), ctx->prior_table.size()))) return bail(rc);
@@ -1889,7 +2031,7 @@ int sl_msampler_sweep(sl_ctx* ctx, int32_t first, int32_t n_chains, const int32_
       ctx->launches += msweep_kernels(ctx, n_meioses) - 1;   // one counted by Prof
       CK(launch_msampler(P, ctx->d_dg, first, n_chains, ctx->d_mlist, 0, n_meioses, ctx->d_u, ucs, 0, 0, nullptr, 0,
                        ctx->d_raw, ctx->d_raw32, ctx->d_fb, ctx->d_badc, ctx->d_maps, ctx->d_status, ctx->ms_threads,
-                       ctx->sampler_precision == SL_SAMPLER_EXACT, ctx->stream, nullptr, ctx->d_mu, msampler_pairs(ctx)));
+                       ctx->sampler_precision == SL_SAMPLER_EXACT, ctx->stream, nullptr, ctx->d_mu, ctx->n_chains, ctx->sweep_load));
     }
     return sl_synchronize(ctx);
 }
@@ -2048,6 +2190,23 @@ int sl_problem_legal_masks(const sl_problem_desc* d, uint8_t* out) {
     int bad = -1;
     if (!genotype_elimination(d, legal, &bad)) return fail(nullptr, SL_EINVAL, "genotypes inconsistent at locus %d", bad);
     std::memcpy(out, legal.data(), legal.size());
+    return SL_OK;
+}
+
+int sl_problem_meiosis_flips(const sl_problem_desc* d, uint8_t* out) {
+    sl_ctx* ctx = nullptr;
+    int rc = check_desc(d);
+    if (rc) return rc;
+    if (!out) return fail(ctx, SL_EINVAL, "null argument");
+    const int N = d->n_members, M = d->n_markers, nm = 2 * (N - d->n_founders), words = (M + 31) / 32;
+    std::vector<uint8_t> geno((size_t)M * N);
+    for (size_t i = 0; i < geno.size(); ++i) geno[i] = d->typed[i % N] ? d->genotypes[i] & 3 : 0;
+    const std::vector<uint32_t> mf = meiosis_flips(d, geno, words);
+    for (int m = 0; m < nm; ++m)
+        for (int l = 0; l < M; ++l) {
+            const uint32_t* w = mf.data() + (size_t)m * 2 * words + (l >> 5);
+            out[(size_t)m * M + l] = (uint8_t)((w[0] >> (l & 31) & 1) | (w[words] >> (l & 31) & 1) << 1);
+        }
     return SL_OK;
 }
 
@@ -2854,7 +3013,7 @@ static cudaError_t capture_chain_body(sl_ctx* ctx, int c, cudaGraph_t body, cuda
     void* fb = exact ? (void*)((double*)ctx->d_fb + (size_t)c * 2 * M) : (void*)((float*)ctx->d_fb + (size_t)c * 2 * M);
     e = launch_msampler(P, ctx->d_dg, c, 1, ctx->d_morder + (size_t)c * nm, nm, nm, nullptr, 0, 0, 0, nullptr, 0, raw,
                         ctx->d_raw32 + (size_t)c * 2 * M, fb, ctx->d_badc + c, ctx->d_maps + (size_t)c * M,
-                        ctx->d_status, ctx->ms_threads, exact ? 1 : 0, s2, key, ctx->d_mu + (size_t)c * M, msampler_pairs(ctx));
+                        ctx->d_status, ctx->ms_threads, exact ? 1 : 0, s2, key, ctx->d_mu + (size_t)c * M, ctx->n_chains, ctx->sweep_load);
     e2 = cudaStreamEndCapture(s2, &sw[1]);
     if (e != cudaSuccess || (e = e2) != cudaSuccess) return e;
     // scoring of chain c into its own table
@@ -2904,7 +3063,7 @@ static int prepare_run_graph(sl_ctx* ctx) {
     CK(cudaMemsetAsync(ctx->d_sel, 0, (size_t)C, ctx->stream));
     CK(launch_msampler(P, ctx->d_dg, 0, C, ctx->d_morder, nm, 0, nullptr, 0, 0, 0, ctx->d_sel, 2, ctx->d_raw,
                        ctx->d_raw32, ctx->d_fb, ctx->d_badc, ctx->d_maps, ctx->d_status, ctx->ms_threads, exact ? 1 : 0,
-                       ctx->stream, ctx->d_keys, ctx->d_mu, msampler_pairs(ctx)));
+                       ctx->stream, ctx->d_keys, ctx->d_mu, ctx->n_chains, ctx->sweep_load));
     CK(ls_launch(ctx, 0, C, ctx->d_even, (int)ctx->even.size(), nullptr, 0, 0, 0, 0, ctx->d_sel, 2,
                        ctx->stream, ctx->d_keys));
     // the scoring kernel is fixed in the graph: time the candidates now if needed
@@ -3169,7 +3328,7 @@ static int build_ms_graph(sl_ctx* ctx) {
     CK(launch_set_key(ctx->d_key, 0, 0, ctx->stream));
     CK(launch_msampler(P, ctx->d_dg, 0, C, ctx->d_morder, nm, 0, nullptr, 0, 0, 0, ctx->d_sel, 2, ctx->d_raw,
                        ctx->d_raw32, ctx->d_fb, ctx->d_badc, ctx->d_maps, ctx->d_status, ctx->ms_threads, exact ? 1 : 0,
-                       ctx->stream, ctx->d_key, ctx->d_mu, msampler_pairs(ctx)));
+                       ctx->stream, ctx->d_key, ctx->d_mu, ctx->n_chains, ctx->sweep_load));
     CK(cudaStreamSynchronize(ctx->stream));
     while ((int)ctx->cap_streams.size() < C + 1) {
         cudaStream_t st;
@@ -3191,7 +3350,7 @@ static int build_ms_graph(sl_ctx* ctx) {
         err = launch_msampler(P, ctx->d_dg, c, 1, ctx->d_morder + (size_t)c * nm, nm, nm, nullptr, 0, 0, 0,
                               ctx->d_sel + c, 0, raw, ctx->d_raw32 + (size_t)c * 2 * M, fb, ctx->d_badc + c,
                               ctx->d_maps + (size_t)c * M, ctx->d_status, ctx->ms_threads, exact ? 1 : 0, sc,
-                              ctx->d_key, ctx->d_mu + (size_t)c * M, msampler_pairs(ctx));
+                              ctx->d_key, ctx->d_mu + (size_t)c * M, ctx->n_chains, ctx->sweep_load);
         if (err != cudaSuccess) break;
         err = cudaEventRecord(ctx->cap_events[c], sc);
         if (err != cudaSuccess) break;
@@ -3215,6 +3374,7 @@ static int build_ms_graph(sl_ctx* ctx) {
 static void account_span(sl_ctx* ctx, const sl_run_options* o, int first, int end) {
     const int C = ctx->n_chains, nm = (int)ctx->meioses.size();
     const int cold = scored_chains(ctx);
+    const int64_t m_kernels = msweep_kernels(ctx, nm);
     int64_t kernels = 1;   // init
     for (int it = first; it < end; ++it) {
         const bool score = it >= o->burnin && it % o->scoring_period == 0;
@@ -3225,7 +3385,7 @@ static void account_span(sl_ctx* ctx, const sl_run_options* o, int first, int en
         for (int c = 0; c < C; ++c) {
             const uint64_t hi = ((uint64_t)c << 40) ^ ((uint64_t)it << 4) ^ 7u;
             const bool is_l = host_philox_u01(o->seed, hi, 0) < o->lsampler_prob;
-            kernels += 2 + (is_l ? 2 : msweep_kernels(ctx, nm)) + (score && ctx->temps[c] == 1.0 ? 2 : 0);
+            kernels += 2 + (is_l ? 2 : m_kernels) + (score && ctx->temps[c] == 1.0 ? 2 : 0);
         }
     }
     ctx->launches += kernels;
@@ -3420,7 +3580,24 @@ int sl_batch_create(sl_ctx* const* ctxs, int32_t n, sl_batch** out) {
     return SL_OK;
 }
 
+// While a batch's graph is captured its contexts' sweeps are shaped for all
+// of the batch's chains running at once.
+namespace {
+struct BatchLoad {
+    sl_batch* b;
+    explicit BatchLoad(sl_batch* b_) : b(b_) {
+        int n = 0;
+        for (sl_ctx* c : b->ctxs) n += c->n_chains;
+        for (sl_ctx* c : b->ctxs) c->sweep_load = n;
+    }
+    ~BatchLoad() {
+        for (sl_ctx* c : b->ctxs) c->sweep_load = c->n_chains;
+    }
+};
+}  // namespace
+
 static int build_batch_graph(sl_batch* b) {
+    const BatchLoad load(b);
     b->ls_epochs.clear();
     for (sl_ctx* c : b->ctxs) {
         int rc = prepare_run_graph(c);
@@ -3455,6 +3632,7 @@ static int build_batch_graph(sl_batch* b) {
 // contexts share the run's spurts; the first context's step decides whether
 // the loop runs again.
 static int build_batch_mc3_graph(sl_batch* b) {
+    const BatchLoad load(b);
     b->mc3_epochs.clear();
     for (sl_ctx* c : b->ctxs) {
         int rc = prepare_run_graph(c);

@@ -48,6 +48,11 @@ struct ProblemDev {
     const uint16_t* typ_cnt;             // [M] typed members per locus
     const uint16_t* typ_nhet;            // [M] heterozygotes per locus
     const uint8_t* typed;                // [N]
+    const uint32_t* mflip;               // [2 Nnf meioses][2][mflip_words]: bit l of the first mask: toggling the meiosis
+                                         // at locus l leaves the founder-allele likelihood as it is, of the second: makes
+                                         // it zero, whatever the rest of a legal graph (meiosis_flips, sl_host.cc); null
+                                         // in the exact mode
+    int32_t mflip_words;                 // ceil(M / 32)
     const double* prior;                 // [M][4 genotype codes][4 states]
     const double* theta;                 // [M-1]
     const double* partial;               // [M-1]

@@ -12,7 +12,9 @@
 //                            founder-allele graph with one meiosis toggled
 //                            (exact mode, and fast mode past the warp form's
 //                            shared-memory limit).
-//  * fag_warp_kernel<G>   -- the same in lane groups of G (fast mode).
+//  * msweep_kernel<G>     -- fast mode: a chain's whole M-sweep by one cluster.
+//  * fag_warp_kernel<G>   -- fast-mode likelihoods in lane groups of G (chains
+//                            whose share of loci does not fit a cluster).
 //  * ffbs_kernel<T>       -- forward filter / backward sample of one meiosis,
 //                            one warp per chain, in the reference's order.
 //  * ffbs_scan_kernel     -- the same as block-wide scans (fast mode).
@@ -36,6 +38,7 @@
 // FP64 arithmetic on decision paths uses __dmul_rn/__dadd_rn/__ddiv_rn so no
 // multiply-add is contracted and the doubles match the reference's.
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <float.h>
 #include <stdint.h>
@@ -49,6 +52,8 @@
 #include "sl_philox.cuh"
 
 namespace sl {
+
+namespace cg = cooperative_groups;
 
 // Raises a kernel's dynamic shared-memory limit on the current device when a
 // launch needs more than it was given so far.  The attribute is per device
@@ -1241,6 +1246,7 @@ __global__ void __launch_bounds__(128) fag_kernel(ProblemDev P, uint32_t* dg, in
 //      gives log2 of the likelihood.
 // ---------------------------------------------------------------------------
 constexpr int kFagWarpsPerBlock = 8;
+constexpr int kMswThreads = 1024;
 constexpr int kFagRounds = 4;   // rounds of colour propagation along heterozygote edges
 
 __host__ __device__ inline size_t fagw_tables(int N) {
@@ -1338,17 +1344,14 @@ struct LaneGroup {
     __device__ __forceinline__ uint32_t shfl(uint32_t v, int src) const { return __shfl_sync(FULLMASK, v, src, G); }
 };
 
-// One (chain, locus) task by one group of G lanes (32 / G loci per warp, in
-// lockstep: every loop below has the same trip count in all groups except the
-// union loop, which holds no warp primitive).  step < 0 stores the likelihood
-// of the column at meiosis order[0]; step >= 0 the likelihoods at both values
-// of meiosis order[step] (the kept one from the previous step).  A group past
-// the last locus (valid false) works on locus 0 and stores nothing.
+// log2 of the genotypes' likelihood at locus lc given the column `col` with
+// meiosis `flip` toggled (-1: as it is), by one group of G lanes (32 / G loci
+// per warp, in lockstep: every loop below has the same trip count in all
+// groups except the union loop, which holds no warp primitive); all lanes of
+// the group return it.
 template <int G, typename E>
-__device__ __forceinline__ void fagw_task(const ProblemDev& P, const FagwTables& tab, unsigned char* wbase,
-                                          const uint32_t* dg, int chain, int cr, int l, bool valid,
-                                          const int32_t* ord, int step, float* rawbuf, float* raw32, uint8_t* badc,
-                                          int* status) {
+__device__ __forceinline__ float fagw_like(const ProblemDev& P, const FagwTables& tab, unsigned char* wbase,
+                                           const uint32_t* col, int chain, int lc, int flip, int* status) {
     const LaneGroup<G> grp;
     const int N = P.N, F = P.F, nfa = 2 * F, M = P.M, gl = grp.gl;
     const uint2* s_lvl = tab.lvl;
@@ -1358,9 +1361,6 @@ __device__ __forceinline__ void fagw_task(const ProblemDev& P, const FagwTables&
     int* fl = (int*)(Lb + nfa);                                       // [2F] bit0 used, bit1 fixed A, bit2 fixed B
     int* cnt = fl + nfa;                                              // [2F] per component: counts, forbidden colourings
     uint16_t* typ = (uint16_t*)(wbase + fagw_typ_offset(N, F, (int)sizeof(E)));   // [N] the locus's typed members
-    const int lc = valid ? l : 0;
-    const uint32_t* col = dg + ((size_t)chain * M + lc) * P.W;
-    float* raw = rawbuf + (size_t)cr * 2 * M;
     // the task's global reads issued together: the column's words (lane w of
     // the group holds word w, read by shuffles), the allele frequencies'
     // log2, and the locus's typed members (member << 2 | genotype code,
@@ -1373,19 +1373,6 @@ __device__ __forceinline__ void fagw_task(const ProblemDev& P, const FagwTables&
     const float2 lfreq = P.c_lfreq[(size_t)chain * M + lc];
     for (int q = gl; q < (ntyp + 7) >> 3; q += G) cp_async16(typ + 8 * q, P.typ_ent + t0 + 8 * q);
     cp_async_commit();
-    auto cbit = [&](int b) -> int {
-        const uint32_t w = wreg ? grp.shfl(cw, b >> 5) : col[b >> 5];
-        return (int)((w >> (b & 31)) & 1u);
-    };
-    int flip = -1, tb = 0;
-    float keep = 0.f;
-    if (step >= 0) {
-        const int m = ord[step];
-        const int last = ord[step > 0 ? step - 1 : 0];
-        tb = cbit(m);
-        keep = raw[2 * lc + cbit(last)];
-        flip = m;
-    }
     // 1. founder alleles, one generation level at a time
     for (int q = gl; q < s_off[1]; q += G) {
         const int pid = (int)s_lvl[q].x;
@@ -1421,13 +1408,18 @@ __device__ __forceinline__ void fagw_task(const ProblemDev& P, const FagwTables&
     }
     cp_async_wait_all();   // this lane's copies of the list; the barrier makes the group's visible
     __syncwarp();
+    int clash = 0;
     for (int x = nhet + gl; x < ntyp; x += G) {
         const int ent = typ[x], i = ent >> 2, g = ent & 3;
         const int bits = g == G_HOMOZ_A ? 3 : 5;   // used, fixed A / fixed B
-        atomicOr(&fl[e[2 * i]], bits);
-        atomicOr(&fl[e[2 * i + 1]], bits);
+        const int b0 = atomicOr(&fl[e[2 * i]], bits) | bits, b1 = atomicOr(&fl[e[2 * i + 1]], bits) | bits;
+        clash |= (b0 & 6) == 6 || (b1 & 6) == 6;
     }
     __syncwarp();
+    // a founder allele fixed to both colours: the likelihood is zero, and the
+    // components need not be worked out (most evaluated toggles end here)
+    clash = grp.any(clash);
+    if (__all_sync(FULLMASK, clash)) return -INFINITY;
     // 3. components of the heterozygote edges with parities: a lock-free
     // union-find forest in Lb (2 * parent + parity to the parent), each lane
     // joining its edges by hooking the larger root under the smaller with a
@@ -1457,7 +1449,7 @@ __device__ __forceinline__ void fagw_task(const ProblemDev& P, const FagwTables&
         __syncwarp();
         if (!__any_sync(FULLMASK, changed)) break;   // the whole warp, as its groups share the loop
     }
-    int bad = 0;
+    int bad = clash;
     for (int q = gl; q < nhet; q += G) {
         const int i = typ[q] >> 2;   // the heterozygotes lead the list
         const int u = e[2 * i], v = e[2 * i + 1];
@@ -1539,8 +1531,32 @@ __device__ __forceinline__ void fagw_task(const ProblemDev& P, const FagwTables&
     }
     zero = grp.any(zero);
     for (int dd = G / 2; dd >= 1; dd >>= 1) sum += __shfl_xor_sync(FULLMASK, sum, dd);
-    const float lk = (bad || zero) ? -INFINITY : sum;
-    if (gl == 0 && valid) {
+    __syncwarp();
+    return (bad || zero) ? -INFINITY : sum;
+}
+
+// One (chain, locus) task by one group of G lanes: step < 0 stores the
+// likelihood of the column at meiosis order[0]; step >= 0 the likelihoods at
+// both values of meiosis order[step] (the kept one from the previous step).
+// A group past the last locus (valid false) works on locus 0 and stores
+// nothing.
+template <int G, typename E>
+__device__ __forceinline__ void fagw_task(const ProblemDev& P, const FagwTables& tab, unsigned char* wbase,
+                                          const uint32_t* dg, int chain, int cr, int l, bool valid,
+                                          const int32_t* ord, int step, float* rawbuf, float* raw32, uint8_t* badc,
+                                          int* status) {
+    const int M = P.M, lc = valid ? l : 0;
+    const uint32_t* col = dg + ((size_t)chain * M + lc) * P.W;
+    float* raw = rawbuf + (size_t)cr * 2 * M;
+    int flip = -1, tb = 0;
+    float keep = 0.f;
+    if (step >= 0) {
+        flip = ord[step];
+        tb = dgbit(col, flip);
+        keep = raw[2 * lc + dgbit(col, ord[step > 0 ? step - 1 : 0])];
+    }
+    const float lk = fagw_like<G, E>(P, tab, wbase, col, chain, lc, flip, status);
+    if ((threadIdx.x & (G - 1)) == 0 && valid) {
         if (step < 0) {
             raw[2 * l + dgbit(col, ord[0])] = lk;
             if (lk == -INFINITY) {
@@ -1713,6 +1729,42 @@ __device__ __forceinline__ void mat_mul_left(float& p00, float& p01, float& p10,
     p00 = n00; p01 = n01; p10 = n10; p11 = n11;
 }
 
+// p <- diag(q) R(t) p, one locus's factor of the filter product
+__device__ __forceinline__ void filter_product(float q0, float q1, float t, float& p00, float& p01, float& p10,
+                                               float& p11) {
+    const float a = 1.f - t;
+    const float n00 = q0 * (a * p00 + t * p10), n01 = q0 * (a * p01 + t * p11);
+    const float n10 = q1 * (t * p00 + a * p10), n11 = q1 * (t * p01 + a * p11);
+    p00 = n00; p01 = n01; p10 = n10; p11 = n11;
+}
+
+// one locus of the filter from the vector (v0, v1) entering it
+__device__ __forceinline__ void filter_locus(float q0, float q1, float t, float v0, float v1, float& f0, float& f1) {
+    const float a = 1.f - t;
+    f0 = q0 * (a * v0 + t * v1);
+    f1 = q1 * (t * v0 + a * v1);
+    const float tot = f0 + f1;
+    if (tot > 0.f) { const float inv = 1.f / tot; f0 *= inv; f1 *= inv; }
+    // keep the reference's exact zeros: a zero likelihood stays zero
+    if (q0 == 0.f) f0 = 0.f;
+    if (q1 == 0.f) f1 = 0.f;
+}
+
+// a locus's decision map from its filtered pair (both non-zero) and its draw;
+// t: the recombination fraction to the locus above (last: none above)
+__device__ __forceinline__ int locus_map(float f0, float f1, double u, bool last, float t) {
+    if (last) {
+        const int v = (u < (double)(f0 / (f0 + f1))) ? 0 : 1;
+        return v | (v << 1);
+    }
+    const float a = 1.f - t;
+    const float x0 = f0 * a, y0 = f1 * t;   // next = 0
+    const float x1 = f0 * t, y1 = f1 * a;   // next = 1
+    const int d0 = (u < (double)(x0 / (x0 + y0))) ? 0 : 1;
+    const int d1 = (u < (double)(x1 / (x1 + y1))) ? 0 : 1;
+    return d0 | (d1 << 1);
+}
+
 // Fast-mode forward filter and backward sampling of one meiosis over all loci,
 // one block per chain (meiosis_sampler.cc:123-203 restated as scans): each
 // thread owns a run of L = ceil(M / T) loci.
@@ -1767,11 +1819,7 @@ __device__ __forceinline__ void ffbs_scan_chain(const ProblemDev& P, uint32_t* d
     // chunk product P = A_{s1-1} ... A_{s0} (A_0 = diag(r_0)); an empty chunk is the identity
     float p00 = 1.f, p01 = 0.f, p10 = 0.f, p11 = 1.f;
     for (int i = s0; i < s1; ++i) {
-        const float q0 = rq(2 * i), q1 = rq(2 * i + 1);
-        const float t = tof(i), a = 1.f - t;
-        const float n00 = q0 * (a * p00 + t * p10), n01 = q0 * (a * p01 + t * p11);
-        const float n10 = q1 * (t * p00 + a * p10), n11 = q1 * (t * p01 + a * p11);
-        p00 = n00; p01 = n01; p10 = n10; p11 = n11;
+        filter_product(rq(2 * i), rq(2 * i + 1), tof(i), p00, p01, p10, p11);
         // each pair is scaled to a maximum of 1, so 8 steps cannot underflow
         if (((i - s0) & 7) == 7) mat_norm(p00, p01, p10, p11);
     }
@@ -1818,14 +1866,8 @@ __device__ __forceinline__ void ffbs_scan_chain(const ProblemDev& P, uint32_t* d
     }
     int cnt = 0;
     for (int i = s0; i < s1; ++i) {
-        const float q0 = rq(2 * i), q1 = rq(2 * i + 1);
-        const float t = tof(i), a = 1.f - t;
-        float f0 = q0 * (a * v0 + t * v1), f1 = q1 * (t * v0 + a * v1);
-        const float tot = f0 + f1;
-        if (tot > 0.f) { const float inv = 1.f / tot; f0 *= inv; f1 *= inv; }
-        // keep the reference's exact zeros: a zero likelihood stays zero
-        if (q0 == 0.f) f0 = 0.f;
-        if (q1 == 0.f) f1 = 0.f;
+        float f0, f1;
+        filter_locus(rq(2 * i), rq(2 * i + 1), tof(i), v0, v1, f0, f1);
         fb[2 * i] = f0;
         fb[2 * i + 1] = f1;
         cnt += (f0 != 0.f && f1 != 0.f);
@@ -1864,17 +1906,7 @@ __device__ __forceinline__ void ffbs_scan_chain(const ProblemDev& P, uint32_t* d
             }
             const double u = ubuf[ub++];
             ++idx;
-            if (i == M - 1) {
-                const int v = (u < (double)(f0 / (f0 + f1))) ? 0 : 1;
-                dmap = v | (v << 1);
-            } else {
-                const float t = tof(i + 1), a = 1.f - t;
-                const float x0 = f0 * a, y0 = f1 * t;   // next = 0
-                const float x1 = f0 * t, y1 = f1 * a;   // next = 1
-                const int d0 = (u < (double)(x0 / (x0 + y0))) ? 0 : 1;
-                const int d1 = (u < (double)(x1 / (x1 + y1))) ? 0 : 1;
-                dmap = d0 | (d1 << 1);
-            }
+            dmap = locus_map(f0, f1, u, i == M - 1, i == M - 1 ? 0.f : tof(i + 1));
         }
         maps[i] = (uint8_t)dmap;
         gmap = map_compose(dmap, gmap);
@@ -1973,6 +2005,337 @@ int ffbs_scan_threads(int M) {
 // Shared bytes: the scan scratch, then (when staged) the chain's arrays.
 size_t ffbs_scan_scratch(int T) { return (size_t)16 * T + 16 * 32 + 4 * 32 + 4 * 36; }
 size_t ffbs_scan_smem(int M) { return ffbs_scan_scratch(ffbs_scan_threads(M)) + (size_t)6 * 4 * M + (size_t)M + 16; }
+
+// ---------------------------------------------------------------------------
+// Fast-mode M-sweep of one chain by one thread-block cluster.
+//
+// Every meiosis step needs the likelihood of each locus with the meiosis
+// toggled, then a filter and a backward draw along all loci.  As two launches
+// per meiosis (fag_warp_kernel, ffbs_scan_kernel) the step of a 120-member,
+// 2,000-SNP chain took 27 us: two dependent launches and a scan on one SM.
+// Here a cluster of CS blocks keeps the chain for the whole sweep: a block
+// owns the loci of its share of ffbs_scan_kernel's warps, holds their columns
+// (when they fit), current likelihoods and filter state in shared memory, and
+// meets the others three times per meiosis in cluster barriers, to pass on the
+// scans' warp totals through distributed shared memory.  The scans keep that
+// kernel's threads, runs and order of operations (a "virtual" warp v of the
+// chain is warp v - rank * vpb of block rank), so graphs are the same bit for
+// bit, whatever CS.
+//
+// Most toggled likelihoods follow from the genotypes and the current one
+// (P.mflip, built with the context, meiosis_flips in sl_host.cc): where the
+// two founder alleles that the meiosis chooses between are both fixed to one
+// colour by homozygous members above it, or nobody below it is typed, the
+// toggled graph has the same terms in the same places, and its likelihood is
+// the current one; where they are fixed to opposite colours and the
+// transmitted one is known, the toggled graph is impossible.  The rest (about
+// one in 14 with 5% of the genotypes missing) are listed and evaluated by the
+// block's warps (fagw_like).
+//
+// Measured, a sweep of every chain: 400 members, 10,000 SNPs, 8 chains 128 ->
+// 31 ms; 120 members, 2,000 SNPs, 10 chains 5.1 -> 2.8 ms (12 us a meiosis).
+// Bound by the evaluated likelihoods (issue with 32 warps on an SM: half of a
+// 400-member step's 33 us, 40% of a 120-member step), then by waiting for the
+// block with the most of them and by the scans' serial runs.
+// ---------------------------------------------------------------------------
+struct MswShape {
+    int cs;        // blocks per cluster
+    int nw, run;   // virtual warps of the chain, loci per virtual thread
+    int vpb;       // virtual warps per block
+    int nl;        // loci per block
+    int threads;   // per block
+    int staged;    // the columns are kept in shared memory
+    size_t task, xch, loci, cols, bytes;   // shared offsets: tasks' scratch, exchange, per-locus arrays, columns; all bytes
+};
+
+// per-locus arrays of a block: filter pairs (8), current and toggled
+// likelihood, theta (one more) and draw index (4 each), two steps' flip masks,
+// the list of loci to evaluate (2) and the decision maps (1)
+static size_t msw_locus_bytes(int nl) { return al16((size_t)nl * (8 + 4 * 4 + 2 + 1) + 4 + 16 * (size_t)(nl / 32)); }
+
+// Shared memory a block of msweep_kernel may take.
+constexpr size_t kMswSmem = 200 * 1024;
+
+// The shape with up to `cs` blocks per cluster; false when a block's share
+// does not fit its shared memory.  A block has a warp for every four of its
+// loci, where one in 14 is evaluated at a step: with 16 warps for 64 loci (30
+// members, 200 markers) a sweep took 0.40 ms, with 32 0.41; with 32 warps for
+// 640 loci (400 members) 20.4 ms, with 16 26.3.
+static bool msw_shape(const ProblemDev& P, int G, int eb, int cs, MswShape* out) {
+    MswShape s;
+    s.nw = ffbs_scan_threads(P.M) / 32;
+    s.run = (P.M + s.nw * 32 - 1) / (s.nw * 32);
+    if (cs > s.nw) cs = s.nw;
+    s.vpb = (s.nw + cs - 1) / cs;
+    s.cs = (s.nw + s.vpb - 1) / s.vpb;
+    s.nl = s.vpb * 32 * s.run;
+    s.task = fagw_tables(P.N);
+    for (int warps = std::min(kMswThreads / 32, std::max(4, s.nl / 4)); warps >= std::max(4, s.vpb); warps /= 2) {
+        s.threads = 32 * warps;
+        s.xch = s.task + (size_t)warps * (32 / G) * fagw_warp_bytes(P.N, P.F, eb);
+        s.loci = s.xch + 16 * 32 + 4 * 32 + 4 * 32 + 16;
+        s.cols = s.loci + msw_locus_bytes(s.nl);
+        s.bytes = s.cols + al16((size_t)4 * P.W * s.nl);
+        s.staged = s.bytes <= kMswSmem;   // else the columns stay in global memory
+        if (!s.staged) s.bytes = s.cols;
+        *out = s;
+        if (s.bytes <= kMswSmem) return true;
+    }
+    return false;
+}
+
+template <int G, typename E>
+__global__ void __launch_bounds__(kMswThreads, 1) msweep_kernel(ProblemDev P, MswShape sh, uint32_t* dg, int first,
+                                                             const int32_t* order, int64_t ostride, int nm,
+                                                             Draws draws, const uint8_t* sel, int want, int* status) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int cr = blockIdx.y;
+    if (sel && sel[cr] != want) return;   // the whole cluster
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, NT = blockDim.x;
+    const int M = P.M, W = P.W, chain = first + cr;
+    const int nw = sh.nw, L = sh.run;
+    const int lo = rank * sh.nl, nl = max(0, min(M, lo + sh.nl) - lo);
+    const FagwTables tab = fagw_load_tables(P, smem);
+    constexpr int kLoci = 32 / G;   // loci per warp
+    unsigned char* scratch = smem + sh.task + (size_t)(warp * kLoci + lane / G) * fagw_warp_bytes(P.N, P.F, (int)sizeof(E));
+    float4* wmat = (float4*)(smem + sh.xch);   // every virtual warp's filter product
+    int* wcnt = (int*)(wmat + 32);             // its draws (bit 30: an impossible pair somewhere in its block)
+    int* wmap = wcnt + 32;                     // its decision map
+    int* ctl = wmap + 32;                      // [0, 1] loci to evaluate at even and odd steps, [2] impossible pair
+    float2* pr = (float2*)(smem + sh.loci);    // [nl] the step's pair, then the filtered pair
+    float* cur = (float*)(pr + sh.nl);         // [nl] log2 likelihood of the column
+    float* tog = cur + sh.nl;                  // [nl] with the meiosis toggled
+    float* th = tog + sh.nl;                   // [nl + 1] theta to the locus below
+    int* didx = (int*)(th + sh.nl + 1);        // [nl] draws above the locus in its block's run
+    uint32_t* msk = (uint32_t*)(didx + sh.nl);   // [2][2][nl / 32] flip masks of this step and the next
+    uint16_t* list = (uint16_t*)(msk + 4 * (sh.nl / 32));
+    uint8_t* maps = (uint8_t*)(list + sh.nl);
+    uint32_t* gcol = dg + ((size_t)chain * M + lo) * W;
+    uint32_t* col = sh.staged ? (uint32_t*)(smem + sh.cols) : gcol;
+    const int32_t* ord = order + cr * ostride;
+    const int nmw = sh.nl / 32, MW = P.mflip_words;
+    if (sh.staged)
+        for (int i = tid; i < nl * W; i += NT) col[i] = gcol[i];
+    for (int i = tid; i <= nl; i += NT) th[i] = lo + i > 0 && lo + i < M ? P.c_theta_f[(size_t)chain * (M - 1) + lo + i - 1] : 0.f;
+    auto load_masks = [&](int step) {   // both masks of the step's meiosis into its buffer
+        if (step >= nm) return;
+        const uint32_t* src = P.mflip + (size_t)ord[step] * 2 * MW;
+        uint32_t* dst = msk + (step & 1) * 2 * nmw;
+        for (int i = tid; i < 2 * nmw; i += NT) {
+            const int k = i >= nmw, w = (k ? i - nmw : i) + (lo >> 5);
+            dst[i] = w < MW ? src[k * MW + w] : 0u;
+        }
+    };
+    load_masks(0);
+    if (tid < 3) ctl[tid] = 0;
+    __syncthreads();
+    // the likelihood of every column as it is
+    for (int h = warp * kLoci; h < nl; h += (NT >> 5) * kLoci) {
+        const int i = h + lane / G;
+        const bool valid = i < nl;
+        const int q = valid ? i : h;
+        const float lk = fagw_like<G, E>(P, tab, scratch, col + (size_t)q * W, chain, lo + q, -1, status);
+        if ((lane & (G - 1)) == 0 && valid) {
+            cur[i] = lk;
+            if (lk == -INFINITY) {
+                ctl[2] = 1;
+                set_status(status, ST_ILLEGAL_DG);
+            }
+        }
+    }
+    cluster.sync();   // every block runs before the first write to another's shared memory
+    const int vw = rank * sh.vpb + warp;                  // this warp's virtual warp
+    const bool scans = warp < sh.vpb && vw < nw;
+    const int s0 = min(M, (vw * 32 + lane) * L) - lo, s1 = min(M, (vw * 32 + lane + 1) * L) - lo;   // its run of loci
+    for (int j = 0; j < nm; ++j) {
+        const int m = ord[j], mw = m >> 5, mb = m & 31;
+        // the step's pairs: from the genotypes where they decide, else listed
+        const uint32_t* em = msk + (j & 1) * 2 * nmw;
+        for (int i0 = warp * 32; i0 < nl; i0 += NT) {
+            const int i = i0 + lane;
+            bool hard = false;
+            if (i < nl) {
+                const float keep = cur[i];
+                const int tb = (col[(size_t)i * W + mw] >> mb) & 1;
+                const bool same = (em[i0 >> 5] >> lane) & 1, never = (em[nmw + (i0 >> 5)] >> lane) & 1;
+                hard = keep == -INFINITY || !(same || never);
+                tog[i] = same ? keep : -INFINITY;
+                pr[i] = same ? make_float2(1.f, 1.f) : make_float2(tb ? 0.f : 1.f, tb ? 1.f : 0.f);
+            }
+            const unsigned b = __ballot_sync(FULLMASK, hard);
+            int at = 0;
+            if (lane == 0 && b) at = atomicAdd(&ctl[j & 1], __popc(b));
+            at = __shfl_sync(FULLMASK, at, 0);
+            if (hard) list[at + __popc(b & ((1u << lane) - 1u))] = (uint16_t)i;
+        }
+        load_masks(j + 1);
+        __syncthreads();
+        const int nh = ctl[j & 1];
+        if (tid == 0) ctl[(j + 1) & 1] = 0;
+        for (int h = warp * kLoci; h < nh; h += (NT >> 5) * kLoci) {
+            const int k = h + lane / G;
+            const bool valid = k < nh;
+            const int i = list[valid ? k : h];
+            const float lk = fagw_like<G, E>(P, tab, scratch, col + (size_t)i * W, chain, lo + i, m, status);
+            if ((lane & (G - 1)) == 0 && valid) {
+                const float keep = cur[i];
+                const int tb = (col[(size_t)i * W + mw] >> mb) & 1;
+                tog[i] = lk;
+                float r2[2];
+                put_raw32_log2(r2, 0, tb ? lk : keep, tb ? keep : lk);
+                pr[i] = make_float2(r2[0], r2[1]);
+                if (keep == -INFINITY && lk == -INFINITY) {
+                    ctl[2] = 1;
+                    set_status(status, ST_ILLEGAL_DG);
+                }
+            }
+        }
+        __syncthreads();
+        // forward filter: run products, scanned within the warp, the warp totals passed to every block
+        float p00 = 1.f, p01 = 0.f, p10 = 0.f, p11 = 1.f;
+        if (scans) {
+            for (int i = s0; i < s1; ++i) {
+                const float2 q = pr[i];
+                filter_product(q.x, q.y, th[i], p00, p01, p10, p11);
+                // each pair is scaled to a maximum of 1, so 8 steps cannot underflow
+                if (((i - s0) & 7) == 7) mat_norm(p00, p01, p10, p11);
+            }
+            mat_norm(p00, p01, p10, p11);
+            for (int d = 1; d < 32; d <<= 1) {
+                const float o00 = __shfl_up_sync(FULLMASK, p00, d), o01 = __shfl_up_sync(FULLMASK, p01, d);
+                const float o10 = __shfl_up_sync(FULLMASK, p10, d), o11 = __shfl_up_sync(FULLMASK, p11, d);
+                if (lane >= d) {
+                    mat_mul_left(p00, p01, p10, p11, o00, o01, o10, o11);
+                    mat_norm(p00, p01, p10, p11);
+                }
+            }
+            const float4 tot = make_float4(__shfl_sync(FULLMASK, p00, 31), __shfl_sync(FULLMASK, p01, 31),
+                                           __shfl_sync(FULLMASK, p10, 31), __shfl_sync(FULLMASK, p11, 31));
+            if (lane < sh.cs) *cluster.map_shared_rank(&wmat[vw], lane) = tot;
+        }
+        cluster.sync();
+        int cnt = 0, x = 0;
+        if (scans) {
+            float4 w = lane < nw ? wmat[lane] : make_float4(1.f, 0.f, 0.f, 1.f);
+            float4 below = vw > 0 ? wmat[vw - 1] : w;   // the product of the thread below lane 0's
+            for (int d = 1; d < 32; d <<= 1) {
+                const float o00 = __shfl_up_sync(FULLMASK, w.x, d), o01 = __shfl_up_sync(FULLMASK, w.y, d);
+                const float o10 = __shfl_up_sync(FULLMASK, w.z, d), o11 = __shfl_up_sync(FULLMASK, w.w, d);
+                if (lane >= d) {
+                    mat_mul_left(w.x, w.y, w.z, w.w, o00, o01, o10, o11);
+                    mat_norm(w.x, w.y, w.z, w.w);
+                }
+            }
+            if (vw > 0) {
+                const int o = vw - 1;
+                mat_mul_left(p00, p01, p10, p11, __shfl_sync(FULLMASK, w.x, o), __shfl_sync(FULLMASK, w.y, o),
+                             __shfl_sync(FULLMASK, w.z, o), __shfl_sync(FULLMASK, w.w, o));
+                mat_norm(p00, p01, p10, p11);
+            }
+            if (vw > 1) {
+                const int o = vw - 2;
+                mat_mul_left(below.x, below.y, below.z, below.w, __shfl_sync(FULLMASK, w.x, o),
+                             __shfl_sync(FULLMASK, w.y, o), __shfl_sync(FULLMASK, w.z, o),
+                             __shfl_sync(FULLMASK, w.w, o));
+                mat_norm(below.x, below.y, below.z, below.w);
+            }
+            // the vector entering the run: S_{k-1} (1, 1)
+            float v0 = __shfl_up_sync(FULLMASK, __fadd_rn(p00, p01), 1);
+            float v1 = __shfl_up_sync(FULLMASK, __fadd_rn(p10, p11), 1);
+            if (lane == 0) {
+                v0 = vw > 0 ? __fadd_rn(below.x, below.y) : 1.f;
+                v1 = vw > 0 ? __fadd_rn(below.z, below.w) : 1.f;
+            }
+            for (int i = s0; i < s1; ++i) {
+                const float2 q = pr[i];
+                float f0, f1;
+                filter_locus(q.x, q.y, th[i], v0, v1, f0, f1);
+                pr[i] = make_float2(f0, f1);
+                cnt += (f0 != 0.f && f1 != 0.f);
+                v0 = f0;
+                v1 = f1;
+            }
+            // draws consumed by loci in higher runs: a suffix sum
+            x = cnt;
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_down_sync(FULLMASK, x, d);
+                if (lane + d < 32) x += y;
+            }
+            const int tot = __shfl_sync(FULLMASK, x, 0) | (ctl[2] ? 1 << 30 : 0);
+            if (lane < sh.cs) *cluster.map_shared_rank(&wcnt[vw], lane) = tot;
+        }
+        cluster.sync();
+        // draws above this block's loci, and whether any block met an impossible pair (the chain then stays as it is)
+        int above = 0, bad = 0;
+        {
+            const int c = lane < nw ? wcnt[lane] : 0;
+            bad = __any_sync(FULLMASK, c >> 30);
+            // draws of the virtual warps above the block's, then of those above this one within it
+            const int hi = (rank + 1) * sh.vpb;
+            int s = lane >= hi ? c & 0x3fffffff : 0;
+            s = __reduce_add_sync(FULLMASK, s);
+            above = s;
+        }
+        if (bad) break;   // every block of the cluster leaves here together
+        if (scans) {
+            int rel = x - cnt;   // draws above this run in the block
+            for (int v = vw + 1; v < min(nw, (rank + 1) * sh.vpb); ++v) rel += wcnt[v] & 0x3fffffff;
+            for (int i = s1 - 1; i >= s0; --i) {
+                const float2 f = pr[i];
+                didx[i] = rel;
+                rel += f.x != 0.f && f.y != 0.f;
+            }
+        }
+        __syncthreads();
+        for (int i = tid; i < nl; i += NT) {
+            const float2 f = pr[i];
+            int dmap;
+            if (f.x == 0.f) dmap = 3;
+            else if (f.y == 0.f) dmap = 0;
+            else dmap = locus_map(f.x, f.y, draws.get(cr, chain, j, above + didx[i]), lo + i == M - 1, th[i + 1]);
+            maps[i] = (uint8_t)dmap;
+        }
+        __syncthreads();
+        int xm = 2;   // identity: bit0 = 0, bit1 = 1
+        if (scans) {
+            for (int i = s1 - 1; i >= s0; --i) xm = map_compose(maps[i], xm);
+            // suffix composition within the warp
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_down_sync(FULLMASK, xm, d);
+                if (lane + d < 32) xm = map_compose(xm, y);
+            }
+            const int tot = __shfl_sync(FULLMASK, xm, 0);
+            if (lane < sh.cs) *cluster.map_shared_rank(&wmap[vw], lane) = tot;
+        }
+        cluster.sync();
+        if (scans) {
+            // every virtual warp above this one, composed
+            int tail = lane > vw && lane < nw ? wmap[lane] : 2;
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_down_sync(FULLMASK, tail, d);
+                if (lane + d < 32) tail = map_compose(tail, y);
+            }
+            tail = __shfl_sync(FULLMASK, tail, 0);
+            // the state entering this run from above (the run holding locus M - 1 ends in a constant map)
+            int in = __shfl_down_sync(FULLMASK, map_compose(xm, tail), 1);
+            if (lane == 31) in = tail;
+            int sv = in & 1;
+            for (int i = s1 - 1; i >= s0; --i) {
+                sv = (maps[i] >> sv) & 1;
+                const uint32_t w = col[(size_t)i * W + mw];
+                if (sv != (int)((w >> mb) & 1u)) {
+                    col[(size_t)i * W + mw] = w ^ (1u << mb);
+                    cur[i] = tog[i];
+                }
+            }
+        }
+        __syncthreads();
+    }
+    __syncthreads();
+    if (sh.staged)
+        for (int i = tid; i < nl * W; i += NT) gcol[i] = col[i];
+}
 
 // ---------------------------------------------------------------------------
 // Trait peel LOD scorer: one warp per (graph, interval, position).
@@ -3318,14 +3681,86 @@ cudaError_t launch_si_select(const uint32_t* scratch, uint32_t* dg, int first, i
     return cudaGetLastError();
 }
 
+// Lanes per founder-allele graph: two loci per warp (16 lanes each: 17% fewer
+// instructions per locus) when the context holds enough chains to be
+// throughput-bound and a column fits in 16 words (with longer columns the
+// 400-member pedigree's M-sweeps were 16% slower than with 32 lanes).
+static int fagw_lanes(const ProblemDev& P, int chains) { return chains >= 8 && P.W <= 16 ? 16 : 32; }
+
+static const void* msw_kernel(int G, int eb) {
+    return G == 16 ? (eb == 1 ? (const void*)msweep_kernel<16, uint8_t> : (const void*)msweep_kernel<16, uint16_t>)
+                   : (eb == 1 ? (const void*)msweep_kernel<32, uint8_t> : (const void*)msweep_kernel<32, uint16_t>);
+}
+
+static void msw_config(const MswShape& sh, int nchain, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at) {
+    *cfg = cudaLaunchConfig_t{};
+    cfg->gridDim = dim3((unsigned)sh.cs, (unsigned)nchain);
+    cfg->blockDim = dim3((unsigned)sh.threads);
+    cfg->dynamicSmemBytes = sh.bytes;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = (unsigned)sh.cs;
+    at->val.clusterDim.y = 1;
+    at->val.clusterDim.z = 1;
+    cfg->attrs = at;
+    cfg->numAttrs = 1;
+}
+
+// Whether fast M-sweeps run as clusters: the genotypes' masks are there and
+// some shape fits (the component counts are 13-bit fields).
+static bool msw_fits(const ProblemDev& P, int G, int eb) {
+    MswShape sh;
+    return P.mflip && 2 * P.F < 8192 && msw_shape(P, G, eb, 16, &sh);
+}
+
+// The most blocks per cluster (16, 8, 4, 2 or 1) at which `load` chains'
+// clusters are all resident, by the occupancy calculator; the fewest that fit
+// when none is.  A sweep of the 400-member, 10,000-SNP pedigree took 20.4,
+// 30.8 and 48.4 ms with 16, 8 and 4 blocks for one chain, 101, 77 and 49 ms
+// for 32 chains; of the 120-member one 2.2, 2.4 and 3.2 ms for one, 31, 15 and
+// 7.8 ms (6.7 with 2 blocks) for 80 chains.
+static cudaError_t msw_choose(const ProblemDev& P, int G, int eb, int load, MswShape* out) {
+    const void* mk = msw_kernel(G, eb);
+    cudaError_t e = cudaFuncSetAttribute(mk, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    for (int cs = 16; cs >= 1 && e == cudaSuccess; cs /= 2) {
+        MswShape sh;
+        if (!msw_shape(P, G, eb, cs, &sh)) break;
+        *out = sh;
+        if ((e = ensure_smem(mk, sh.bytes)) != cudaSuccess) break;
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at;
+        msw_config(sh, load, &cfg, &at);
+        int active = 0;
+        if ((e = cudaOccupancyMaxActiveClusters(&active, mk, &cfg)) == cudaSuccess && active >= load) break;
+    }
+    return e;
+}
+
+// Kernels of one fast M-sweep of nm meioses in a context of `chains` chains.
+int64_t msweep_launches(const ProblemDev& P, int chains, int nm) {
+    return msw_fits(P, fagw_lanes(P, chains), fagw_label_bytes(P.F)) ? 1 : 1 + 2 * (int64_t)nm;
+}
+
 template <typename IX, typename PP>
 static cudaError_t launch_msampler_t(const ProblemDev& P, uint32_t* dg, int first, int nchain, const int32_t* meioses,
                                      int64_t mstride, int nm, const double* u, int64_t ucs, uint64_t seed,
                                      uint64_t iter, const uint8_t* sel, int want, typename PP::T* raw, float* raw32,
                                      void* fb, uint8_t* badc, uint8_t* maps, int* status, int fag_threads, int exact,
-                                     cudaStream_t s, const uint64_t* key, double* ubuf, int pairs) {
+                                     cudaStream_t s, const uint64_t* key, double* ubuf, int chains, int load) {
     const int fast = exact ? 0 : 1;
     Draws d{u, ucs, P.M, seed, iter, 2, key};
+    const int G = fagw_lanes(P, chains), eb = fagw_label_bytes(P.F);
+    if (!exact && msw_fits(P, G, eb)) {
+        MswShape sh;
+        cudaError_t e = msw_choose(P, G, eb, std::max(load, nchain), &sh);
+        if (e != cudaSuccess) return e;
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at;
+        msw_config(sh, nchain, &cfg, &at);
+        cfg.stream = s;
+        void* args[] = {(void*)&P, (void*)&sh, (void*)&dg, (void*)&first, (void*)&meioses, (void*)&mstride,
+                        (void*)&nm, (void*)&d, (void*)&sel, (void*)&want, (void*)&status};
+        return cudaLaunchKernelExC(&cfg, msw_kernel(G, eb), args);
+    }
     cudaError_t e0 = cudaMemsetAsync(badc, 0, (size_t)nchain, s);
     if (e0 != cudaSuccess) return e0;
     const size_t smem = fag_block_bytes(P.N, P.F, fag_threads, fast);
@@ -3348,13 +3783,6 @@ static cudaError_t launch_msampler_t(const ProblemDev& P, uint32_t* dg, int firs
     const int grid = (int)((ntask + fag_threads - 1) / fag_threads);
     // fast mode: one warp per (chain, locus), else the thread-per-locus kernel
     // in log2 (component counts are 13-bit fields)
-    // two loci per warp (16 lanes each: 17% fewer instructions per locus, 30%
-    // longer per launch) when the caller asks for throughput and a column
-    // fits in 16 words (with longer columns read from global memory and the
-    // block's shared memory doubled, the 400-member pedigree's M-sweeps were
-    // 16% slower than with 32 lanes)
-    const int G = pairs && P.W <= 16 ? 16 : 32;
-    const int eb = fagw_label_bytes(P.F);
     const size_t wsm = fagw_block_bytes(P.N, P.F, G, eb);
     const bool warp_like = !exact && wsm <= 200 * 1024 && 2 * P.F < 8192;
     const void* fk = G == 16 ? (eb == 1 ? (const void*)fag_warp_kernel<16, uint8_t> : (const void*)fag_warp_kernel<16, uint16_t>)
@@ -3416,25 +3844,25 @@ cudaError_t launch_msampler(const ProblemDev& P, uint32_t* dg, int first, int nc
                             int64_t mstride, int nm, const double* u, int64_t ucs, uint64_t seed, uint64_t iter,
                             const uint8_t* sel, int want, double* raw64, float* raw32, void* fb, uint8_t* badc,
                             uint8_t* maps, int* status, int fag_threads, int exact, cudaStream_t s,
-                            const uint64_t* key, double* ubuf, int pairs) {
+                            const uint64_t* key, double* ubuf, int chains, int load) {
     // the fast mode keeps log2 likelihoods as floats in the first half of the raw buffer
     float* rawl = (float*)raw64;
     if (2 * P.F <= 255) {
         if (exact)
             return launch_msampler_t<uint8_t, ProbExact>(P, dg, first, nchain, meioses, mstride, nm, u, ucs, seed,
                                                          iter, sel, want, raw64, raw32, fb, badc, maps, status,
-                                                         fag_threads, exact, s, key, ubuf, pairs);
+                                                         fag_threads, exact, s, key, ubuf, chains, load);
         return launch_msampler_t<uint8_t, ProbLog2>(P, dg, first, nchain, meioses, mstride, nm, u, ucs, seed, iter,
                                                     sel, want, rawl, raw32, fb, badc, maps, status, fag_threads,
-                                                    exact, s, key, ubuf, pairs);
+                                                    exact, s, key, ubuf, chains, load);
     }
     if (exact)
         return launch_msampler_t<uint16_t, ProbExact>(P, dg, first, nchain, meioses, mstride, nm, u, ucs, seed, iter,
                                                       sel, want, raw64, raw32, fb, badc, maps, status, fag_threads,
-                                                      exact, s, key, ubuf, pairs);
+                                                      exact, s, key, ubuf, chains, load);
     return launch_msampler_t<uint16_t, ProbLog2>(P, dg, first, nchain, meioses, mstride, nm, u, ucs, seed, iter, sel,
                                                  want, rawl, raw32, fb, badc, maps, status, fag_threads, exact, s,
-                                                 key, ubuf, pairs);
+                                                 key, ubuf, chains, load);
 }
 
 size_t fag_smem(int N, int F, int threads, int fast) { return fag_block_bytes(N, F, threads, fast); }

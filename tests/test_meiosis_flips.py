@@ -1,0 +1,108 @@
+"""The fast M-sampler's rule on which toggled likelihoods it evaluates
+(sl_problem_meiosis_flips) against the founder-allele-graph likelihood of the
+C restatement, and its clusters against one another."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from oracle import port
+from swiftlink_gb300 import api, pedigree, synth
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _built():
+    from swiftlink_gb300 import build
+    build.build()
+    port.build()
+
+
+def family(members, loops, markers, untyped, missing, seed):
+    """A looped pedigree with whole members and single genotypes untyped, and a legal graph."""
+    gens = 3 + (members >= 25) + (members >= 90)
+    spec = synth.WorkloadSpec(n_members=members, generations=gens, loops=loops, affected=3, markers=markers,
+                              spacing_cm=0.5, maf=(0.05, 0.5), missing_all=missing, disease_cm=0.4)
+    for k in range(20):   # the first seed whose topology has the shape
+        try:
+            w = synth.make_workload(1, seed=seed + 1000 * k, spec=spec)
+            break
+        except RuntimeError:
+            continue
+    g = pedigree.problem_from_workload(w)
+    rng = np.random.default_rng(seed)
+    out = rng.random(g["N"]) < untyped
+    g["genotypes"][:, out] = 0
+    g["typed"] = (g["genotypes"] != 0).any(axis=0).astype(np.uint8)
+    return g
+
+
+def flips(g):
+    prob = api.Problem.from_arrays(g, with_legal=False)
+    desc = prob.desc()
+    out = np.zeros((2 * (g["N"] - g["F"]), g["M"]), np.uint8)
+    assert api.lib().sl_problem_meiosis_flips(ctypes.byref(desc), out.ctypes.data_as(ctypes.c_void_p)) == 0
+    return out
+
+
+# pedigree sizes, loops (inbred members and marriages between relatives), untyped members, missing genotypes,
+# marker counts on both sides of a mask word
+@pytest.mark.parametrize("members,loops,markers,untyped,missing,seed", [
+    (12, 0, 33, 0.0, 0.0, 1), (25, 1, 64, 0.0, 0.3, 2), (40, 3, 31, 0.3, 0.1, 3), (60, 2, 32, 0.6, 0.05, 4),
+    (110, 4, 40, 0.1, 0.5, 5), (110, 3, 65, 0.0, 0.05, 6)])
+def test_flips_follow_from_the_genotypes(members, loops, markers, untyped, missing, seed):
+    """Every (meiosis, locus) that the rule decides, on two legal graphs (the
+    gene drop's, and one moved away from it by legal toggles): the toggled
+    likelihood is the current one (the same factors; 1e-12 covers their order)
+    or zero."""
+    g = family(members, loops, markers, untyped, missing, seed)
+    rule = flips(g)
+    assert not np.any(rule == 3)
+    P = port.Port(dict(g, legal=np.full((g["M"], g["N"]), 15, np.uint8), trait_prior=np.zeros((g["M"], g["N"], 4))))
+    rng = np.random.default_rng(seed + 100)
+    dg = np.ascontiguousarray(g["dg0"], np.int32)
+    decided = 0
+    for graph in range(2):
+        for l in range(g["M"]):
+            base = P.fag(dg, l)
+            assert base > 0.0
+            for m in rng.permutation(rule.shape[0]):
+                person, par = g["F"] + m // 2, m % 2
+                if graph == 1 and rule[m, l] == 0 and rng.random() < 0.7:
+                    continue
+                dg[l, person, par] ^= 1
+                lk = P.fag(dg, l)
+                if rule[m, l] == 1:
+                    assert abs(lk - base) <= 1e-12 * base, (m, l)
+                elif rule[m, l] == 2:
+                    assert lk == 0.0, (m, l)
+                decided += rule[m, l] != 0
+                if lk > 0.0 and rng.random() < 0.5:
+                    base = lk   # keep the toggle: another legal graph
+                else:
+                    dg[l, person, par] ^= 1
+    assert decided > 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("members,markers,untyped", [(25, 2, 0.0), (25, 63, 0.3), (25, 65, 0.0), (40, 129, 0.2),
+                                                     (60, 1000, 0.0), (110, 2113, 0.1)])
+def test_sweep_is_the_same_whatever_the_cluster(members, markers, untyped):
+    """Contexts of 1, 5 and 7 chains shape their clusters differently from a
+    context of 600 chains' worth of load (a batch), and all sweep chain 0
+    alike, bit for bit; 8 and 40 chains likewise (two graphs per warp there)."""
+    g = family(members, 1, markers, untyped, 0.05, members + markers)
+    nm = min(len(g["meioses"]), 30)
+    prob = api.Problem.from_arrays(g, with_legal=False)
+    u = np.random.default_rng(3).random((nm, markers))
+    got = {}
+    for chains in (1, 5, 7, 8, 40):
+        with api.Context(prob, n_chains=chains, sampler_precision=api.SL_SAMPLER_FAST) as ctx:
+            dg = np.ascontiguousarray(g["dg0"], np.int32)
+            ctx.set_graphs(np.broadcast_to(dg, (chains,) + dg.shape))
+            ctx.msampler_sweep(g["meioses"][:nm], np.broadcast_to(u, (chains,) + u.shape), n_chains=chains)
+            out = ctx.get_graphs()
+        assert all(np.array_equal(out[0], x) for x in out), f"{chains} chains: a chain differs from the first"
+        got[chains] = out[0]
+    assert not np.array_equal(got[1], dg)
+    assert np.array_equal(got[1], got[5]) and np.array_equal(got[1], got[7])
+    assert np.array_equal(got[8], got[40])
