@@ -132,13 +132,18 @@ typedef struct sl_options {
  * rfunction cells allowed by genotype elimination and wins on pedigrees with
  * large cutsets (hundreds of members), the specialised one on smaller ones. */
 #define SL_LS_KERNEL_AUTO 3
-/* GENERIC times 32, 16 and 8 lanes per (chain, locus) task (one, two or four
- * tasks per warp) before the first L-sampler work and keeps the fastest,
- * sharing the choice between contexts of one pedigree size class; these
- * three force one (all forms draw the same graphs). */
+/* GENERIC gives a (chain, locus) task 4 lanes (eight tasks per warp) where the
+ * rfunctions are small (at most 16 cells an operation at the widest locus);
+ * else it times 32, 16, 8 and 4 lanes before the first L-sampler work and
+ * keeps the fastest, sharing the choice between contexts of one pedigree size
+ * class.  These four force one (all forms draw the same graphs).  GENERIC4 fails
+ * sl_create for a peel sequence outside its limits: cutsets of at most 8
+ * members, 16 children per parent peel, every cutset member peeled by a later
+ * operation. */
 #define SL_LS_KERNEL_GENERIC32 4
 #define SL_LS_KERNEL_GENERIC16 5
 #define SL_LS_KERNEL_GENERIC8 6
+#define SL_LS_KERNEL_GENERIC4 7
 
 /* A LOD position whose trait likelihood is 0 (an affected and an unaffected
  * member IBD 2 under a fully penetrant model, for instance) stops the
@@ -470,10 +475,10 @@ int sl_lod_kernel_info(sl_ctx* ctx, int32_t* kernel, double* compile_ms);
 int sl_ls_kernel_info(sl_ctx* ctx, int32_t* kernel, double* compile_ms);
 
 /* The L-sampler autotuner's outcome: the lanes per (chain, locus) task of the
- * generic kernel in use (32, 16 or 8; 0 when the specialised kernel runs) and
- * the timed half-sweep of each candidate in milliseconds, times_ms[0..3] =
- * 32, 16 and 8 lanes and the specialised kernel (0 for a candidate not timed,
- * and for all of them before the first L-sampler work or when a pedigree of
+ * generic kernel in use (32, 16, 8 or 4; 0 when the specialised kernel runs)
+ * and the timed half-sweep of each candidate in milliseconds, times_ms[0..3] =
+ * 32, 16 and 8 lanes and the specialised kernel (4 lanes are timed beside them
+ * and not reported; 0 for a candidate not timed, and for all of them before the first L-sampler work or when a pedigree of
  * the same size class on this device was timed first).  Either pointer may
  * be NULL. */
 int sl_ls_tuning(sl_ctx* ctx, int32_t* lanes, double* times_ms);

@@ -33,10 +33,12 @@ namespace sl {
 size_t lsampler_smem_per_warp(const ProblemDev& P);
 size_t lsampler_smem_shared(const ProblemDev& P);
 int lsampler_resident_tasks(const ProblemDev& P, int wpb);
+size_t quad_arena_per_warp(const ProblemDev& P);
+size_t quad_block_bytes(const ProblemDev& P, int warps);
 cudaError_t launch_lsampler(const ProblemDev& P, uint32_t* dg, int first, int nchain, const int32_t* loci,
                             int nloci, const double* u, int64_t ucs, int64_t uls, uint64_t seed, uint64_t iter,
                             const uint8_t* sel, int want, int* status, cudaStream_t s, int grid_cap, int wpb,
-                            const uint64_t* key = nullptr, int lanes = 32);
+                            const uint64_t* key = nullptr, int lanes = 32, int load = 1, int sms = 1);
 cudaError_t launch_msampler(const ProblemDev& P, uint32_t* dg, int first, int nchain, const int32_t* meioses,
                             int64_t mstride, int nm, const double* u, int64_t ucs, uint64_t seed, uint64_t iter,
                             const uint8_t* sel, int want, double* raw64, float* raw32, void* fb, uint8_t* badc,
@@ -47,7 +49,7 @@ cudaError_t launch_set_key(uint64_t* key, uint64_t seed, uint64_t iter, cudaStre
 cudaError_t launch_lfreq(const double* minor, float2* out, int64_t n, cudaStream_t s);
 cudaError_t launch_si(const ProblemDev& P, uint32_t* dg, int first, int nchain, const int32_t* starts,
                       const double* u, int64_t ucs, uint64_t seed, uint64_t pass, double* weights, int* status,
-                      cudaStream_t s, int wpb, int npass, int64_t pass_stride, int grid_cap);
+                      cudaStream_t s, int wpb, int npass, int64_t pass_stride, int grid_cap, bool quad, int sms);
 cudaError_t launch_si_select(const uint32_t* scratch, uint32_t* dg, int first, int nchain, size_t words,
                              const double* w, double* best, int npass, cudaStream_t s);
 cudaError_t launch_run_init(const RunParams* rp, int64_t* it, int C, cudaStream_t s);
@@ -90,8 +92,12 @@ thread_local std::string g_err;
 const size_t kSmemBudget = 200 * 1024;  // dynamic shared memory a block may use
 }  // namespace
 
-enum { LS_GEN32 = 0, LS_GEN16 = 1, LS_JIT = 2, LS_GEN8 = 3 };
-static int ls_lanes(int choice) { return choice == LS_GEN16 ? 16 : (choice == LS_GEN8 ? 8 : 32); }
+enum { LS_GEN32 = 0, LS_GEN16 = 1, LS_JIT = 2, LS_GEN8 = 3, LS_QUAD = 4 };
+static int ls_lanes(int choice) {
+    return choice == LS_QUAD ? 4 : choice == LS_GEN16 ? 16 : (choice == LS_GEN8 ? 8 : 32);
+}
+constexpr int kQuadWarpTasks = 8, kQuadBlockWarps = 8;   // lsampler_quad_kernel's tasks per warp, most warps per block
+constexpr size_t kQuadArenaBytes = size_t(4) << 30;      // most global memory a context gives its rfunctions
 
 struct sl_ctx {
     int device = 0;
@@ -214,8 +220,9 @@ struct sl_ctx {
     // the L-sampler's kernel and lanes per task: the generic kernel with 32 or
     // 16 lanes, or the specialised one; chosen by timing (ls_tune) unless forced
     bool ls_tune_pending = false;
-    int ls_choice = 0;                          // LS_GEN32, LS_GEN16, LS_GEN8, LS_JIT
-    double ls_tune_ms[4] = {0.0, 0.0, 0.0, 0.0};   // one timed half-sweep with each (0: not timed)
+    int ls_choice = 0;                          // LS_GEN32, LS_GEN16, LS_GEN8, LS_JIT, LS_QUAD
+    bool quad_ok = false;                       // the peel sequence suits the four-lane kernel
+    double ls_tune_ms[5] = {0.0, 0.0, 0.0, 0.0, 0.0};   // one timed half-sweep with each (0: not timed)
     int lod_kernel_sel = SL_LOD_KERNEL_INTERP;   // AUTO while the first scoring has not timed them
     JitLod jit_reg, jit_smem;
     double jit_ms = 0.0;
@@ -259,7 +266,7 @@ static cudaError_t ls_launch(sl_ctx* ctx, int first, int nchain, const int32_t* 
         return jit_ls_launch(ctx->jit_ls, ctx->d_dg, first, nchain, loci, nloci, u, ucs, uls, seed, iter, key, sel,
                              want, ctx->d_status, P.geno, P.prior_f, P.c_theta_f, ctx->sms, s);
     return launch_lsampler(P, ctx->d_dg, first, nchain, loci, nloci, u, ucs, uls, seed, iter, sel, want, ctx->d_status,
-                           s, ctx->ls_grid, ctx->ls_wpb, key, ls_lanes(ctx->ls_choice));
+                           s, ctx->ls_grid, ctx->ls_wpb, key, ls_lanes(ctx->ls_choice), ctx->sweep_load, ctx->sms);
 }
 
 // Takes up a background compile of the specialised L-sampler that has ended:
@@ -349,9 +356,9 @@ static int fail(sl_ctx* c, int code, const char* fmt, ...) {
     } while (0)
 
 // The L-sampler autotuner: times one even-locus half-sweep of every chain
-// with each candidate -- the generic kernel with 32 lanes per (chain, locus)
-// task and with 16 (two tasks per warp), and the specialised kernel when it
-// was built for SL_LS_KERNEL_AUTO -- on a copy of the chains' graphs (the
+// with each candidate -- the generic kernel with 32, 16, 8 and 4 lanes per
+// (chain, locus) task, and the specialised kernel when it was built for
+// SL_LS_KERNEL_AUTO -- on a copy of the chains' graphs (the
 // chains are not touched), and keeps the fastest, as the reference times its
 // launch shapes and locus groupings (gpu_lodscores.cc:541-596,
 // markov_chain.cc:269-311).  Every candidate draws the same graphs, so the
@@ -363,17 +370,52 @@ static int fail(sl_ctx* c, int code, const char* fmt, ...) {
 static std::mutex g_ls_class_mu;
 static std::map<std::tuple<int, int, int, int, int, bool>, int> g_ls_class;
 
+// Whether the four-lane kernel can run: its shared memory, and the global
+// arena (allocated here) with room for a half-sweep of every chain, or for as
+// many warps a chain as kQuadArenaBytes holds.
+template <typename T>
+static int dev_alloc(sl_ctx* ctx, T** p, size_t n);
+static bool quad_ready(sl_ctx* ctx) {
+    ProblemDev& P = ctx->P;
+    if (!ctx->quad_ok || quad_block_bytes(P, 1) > kSmemBudget) return false;
+    const size_t per = quad_arena_per_warp(P);
+    if (!per || P.quad_arena) return true;
+    int64_t warps = ((int64_t)ctx->even.size() + kQuadWarpTasks - 1) / kQuadWarpTasks;
+    warps = std::min<int64_t>(warps, (int64_t)(kQuadArenaBytes / per / ctx->n_chains));
+    warps = std::max<int64_t>(1, (warps + kQuadBlockWarps - 1) / kQuadBlockWarps) * kQuadBlockWarps;
+    uint8_t* a = nullptr;
+    if (dev_alloc(ctx, &a, (size_t)warps * per * ctx->n_chains)) {
+        cudaGetLastError();
+        ctx->err.clear();
+        return false;
+    }
+    P.quad_arena = a;
+    P.quad_warps = warps;
+    return true;
+}
+
 static int ls_tune(sl_ctx* ctx) {
     if (!ctx->ls_tune_pending) return SL_OK;
     ctx->ls_tune_pending = false;
     const ProblemDev& P = ctx->P;
+    const bool quad = quad_ready(ctx);
     const bool jit = ctx->jit_ls.kern != nullptr;
+    // Four lanes per task without a timing where the rfunctions are small (up
+    // to 16 cells an operation at the widest locus): fastest there in every
+    // pedigree and number of chains measured, by 1.3 to 5.5 times (see
+    // lsampler_quad_kernel); wide rfunctions may want a task's cells spread
+    // over more lanes, and are timed.
+    if (quad && !jit && P.ls_arena <= 16 * P.K) {
+        if (ctx->ls_choice != LS_QUAD) ++ctx->ls_epoch;
+        ctx->ls_choice = LS_QUAD;
+        return SL_OK;
+    }
     const auto key = std::make_tuple(ctx->device, P.ls_fast, P.K / 25, P.ls_arena / 128, std::min(ctx->n_chains, 64),
                                      jit);
     if (!jit) {
         std::lock_guard<std::mutex> g(g_ls_class_mu);
         auto it = g_ls_class.find(key);
-        if (it != g_ls_class.end()) {
+        if (it != g_ls_class.end() && (it->second != LS_QUAD || quad)) {
             if (it->second != ctx->ls_choice) ++ctx->ls_epoch;
             ctx->ls_choice = it->second;
             return SL_OK;
@@ -392,6 +434,7 @@ static int ls_tune(sl_ctx* ctx) {
     CK(cudaMemcpyAsync(scratch, ctx->d_dg, sizeof(uint32_t) * words, cudaMemcpyDeviceToDevice, ctx->stream));
     cudaEvent_t a = take_event(ctx), b = take_event(ctx);
     std::vector<int> cand = {LS_GEN32, LS_GEN16, LS_GEN8};
+    if (quad) cand.push_back(LS_QUAD);
     if (jit) cand.push_back(LS_JIT);
     int best = ctx->ls_choice;
     float best_ms = 0.f;
@@ -406,7 +449,7 @@ static int ls_tune(sl_ctx* ctx) {
             else
                 CK(launch_lsampler(P, scratch, 0, C, ctx->d_even, (int)ctx->even.size(), nullptr, 0, 0, 1, 0,
                                    nullptr, 0, ctx->d_status, ctx->stream, ctx->ls_grid, ctx->ls_wpb, nullptr,
-                                   ls_lanes(k)));
+                                   ls_lanes(k), C, ctx->sms));
             if (rep == 1) {
                 CK(cudaEventRecord(b, ctx->stream));
                 CK(cudaEventSynchronize(b));
@@ -691,6 +734,59 @@ static void pack_graphs(const int32_t* src, int n, int N, int F, int M, int W, u
 static void unpack_graphs(const uint32_t* src, int n, int N, int F, int M, int W, int32_t* dst) {
     for_columns((size_t)n * M, (size_t)n * M * N * 8,
                 [&](size_t a, size_t b) { unpack_columns(src, N, F, W, dst, a, b); });
+}
+
+// The peel operations in the four-lane L-sampler's packed form (QuadOp,
+// sl_kernels.cu); false when they do not suit it: cutsets of at most 8
+// members, at most 16 children and 31 previous rfunctions per operation, and
+// every cutset member sampled (peeled by a later operation) before the
+// operation that reads it.
+static bool pack_quad_ops(const sl_problem_desc* d, const std::vector<OpDev>& ops, const std::vector<int32_t>& od,
+                          std::vector<uint32_t>& out, int32_t* tail_words) {
+    const int N = d->n_members, F = d->n_founders, K = (int)ops.size();
+    *tail_words = 0;
+    std::vector<int> peeled(N, -1);
+    for (int k = 0; k < K; ++k) peeled[ops[k].peel] = k;
+    std::vector<uint16_t> tail;
+    for (int k = 0; k < K; ++k) {
+        const OpDev& op = ops[k];
+        const int kids = op.type == CHILD ? 1 : op.type == PARENT ? op.n_child : 0;
+        if (op.c > 8 || kids > 16 || op.n_prev > 31 || out.size() > 65535) return false;
+        tail.push_back((uint16_t)out.size());
+        out.push_back((uint32_t)(op.c | op.type << 4 | op.n_prev << 7 | kids << 12 |
+                                 (op.type == CHILD ? op.mpos << 17 | op.fpos << 21 : 0)));
+        out.push_back((uint32_t)op.peel);
+        const int32_t* cut = od.data() + op.cut_at;
+        for (int q = 0; q < op.c; ++q) {
+            if (peeled[cut[q]] <= k) return false;
+            if (q % 2 == 0) out.push_back((uint32_t)cut[q]);
+            else out.back() |= (uint32_t)cut[q] << 16;
+        }
+        const int32_t* pd = od.data() + op.prev_at;
+        const int32_t* po = od.data() + op.prev_ops_at;
+        for (int j = 0; j < op.n_prev; ++j, pd += 2 + pd[1]) {
+            if (pd[1] > 8) return false;
+            out.push_back((uint32_t)po[j] | (uint32_t)pd[1] << 16);
+            uint32_t keys = 0;
+            for (int q = 0; q < pd[1]; ++q) keys |= (uint32_t)pd[2 + q] << (4 * q);
+            out.push_back(keys);
+        }
+        if (op.type == CHILD) out.push_back((uint32_t)(2 * (op.peel - F)));
+        if (op.type == PARENT)
+            for (int c = 0; c < op.n_child; ++c) {
+                const int32_t* cd = od.data() + op.child_at + 4 * c;
+                out.push_back((uint32_t)(2 * (cd[0] - F)) | (uint32_t)cd[1] << 16 | (uint32_t)cd[2] << 20 |
+                              (uint32_t)cd[3] << 24);
+            }
+    }
+    for (int i = F; i < N; ++i) {
+        tail.push_back((uint16_t)d->mother[i]);
+        tail.push_back((uint16_t)d->father[i]);
+    }
+    if (tail.size() % 2) tail.push_back(0);
+    for (size_t i = 0; i < tail.size(); i += 2) out.push_back(tail[i] | (uint32_t)tail[i + 1] << 16);
+    *tail_words = (int32_t)(tail.size() / 2);
+    return true;
 }
 
 // What a locus's genotypes alone say about toggling a meiosis there
@@ -1551,6 +1647,8 @@ int sl_create(const sl_problem_desc* d, const sl_options* opt, sl_ctx** out) {
     P.marker_trans = std::log(0.5) * (2 * (N - F));
     P.lod_zero_ok = (opt->lod_flags & SL_LOD_ZERO_OK) ? 1 : 0;
     P.ls_fast = opt->sampler_precision == SL_SAMPLER_FAST ? 1 : 0;
+    P.quad_arena = nullptr;
+    P.quad_warps = 0;
     if ((rc = upload(ctx, (int16_t**)&P.mother, mo.data(), N))) return bail(rc);
     if ((rc = upload(ctx, (int16_t**)&P.father, fa.data(), N))) return bail(rc);
     if ((rc = upload(ctx, (uint8_t**)&P.geno, geno.data(), geno.size()))) return bail(rc);
@@ -1707,6 +1805,10 @@ int sl_create(const sl_problem_desc* d, const sl_options* opt, sl_ctx** out) {
     CK(cudaMemset(ctx->d_status, 0, sizeof(int)));
     CK(cudaMemset(ctx->d_acc, 0, sizeof(double) * npos));
     CK(cudaMemset(ctx->d_init, 0, npos));
+    std::vector<uint32_t> qp;
+    ctx->quad_ok = pack_quad_ops(d, ops, od, qp, &P.quad_tail_words);
+    P.quad_prog_words = (int32_t)qp.size();
+    if (ctx->quad_ok && (rc = upload(ctx, (uint32_t**)&P.quad_prog, qp.data(), qp.size()))) return bail(rc);
     ctx->theta_h.assign(d->theta, d->theta + M - 1);
     ctx->minor_h.assign(d->minor_freq, d->minor_freq + M);
     ctx->temps.assign(C, 1.0);
@@ -1774,11 +1876,16 @@ int sl_create(const sl_problem_desc* d, const sl_options* opt, sl_ctx** out) {
         const int req = opt->ls_kernel;
         if (req != SL_LS_KERNEL_GENERIC && req != SL_LS_KERNEL_SPECIALISED && req != SL_LS_KERNEL_BACKGROUND &&
             req != SL_LS_KERNEL_AUTO && req != SL_LS_KERNEL_GENERIC32 && req != SL_LS_KERNEL_GENERIC16 &&
-            req != SL_LS_KERNEL_GENERIC8)
+            req != SL_LS_KERNEL_GENERIC8 && req != SL_LS_KERNEL_GENERIC4)
             return bail(fail(nullptr, SL_EINVAL, "unknown ls_kernel %d", req));
         if (req == SL_LS_KERNEL_GENERIC) ctx->ls_tune_pending = true;   // 32, 16 or 8 lanes per task, by timing
         if (req == SL_LS_KERNEL_GENERIC16) ctx->ls_choice = LS_GEN16;
         if (req == SL_LS_KERNEL_GENERIC8) ctx->ls_choice = LS_GEN8;
+        if (req == SL_LS_KERNEL_GENERIC4) {
+            if (!quad_ready(ctx))
+                return bail(fail(nullptr, SL_EINVAL, "the peel sequence does not suit four lanes per L-sampler task"));
+            ctx->ls_choice = LS_QUAD;
+        }
         if (P.ls_fast && req == SL_LS_KERNEL_BACKGROUND) {
             // the source now (host tables in hand), the compile on a thread started once creation has succeeded
             const JitLsIn in{ops.data(), od.data(), K, N, F, M, P.W, N - F, arena, max_child, d->mother, d->father};
@@ -3793,7 +3900,7 @@ int sl_sequential_imputation(sl_ctx* ctx, int32_t first, int32_t n_chains, const
     CK(cudaMemcpyAsync(d_starts, start_loci, sizeof(int32_t) * n_chains, cudaMemcpyHostToDevice, ctx->stream));
     { Prof pf_(ctx, SL_KERNEL_LSAMPLER);
     CK(launch_si(ctx->P, ctx->d_dg, first, n_chains, d_starts, ctx->d_u, chain_stride, 0, 0, d_w, ctx->d_status,
-                 ctx->stream, ctx->ls_wpb, 1, 0, ctx->ls_grid)); }
+                 ctx->stream, ctx->ls_wpb, 1, 0, ctx->ls_grid, quad_ready(ctx), ctx->sms)); }
     CK(cudaMemcpyAsync(weights, d_w, sizeof(double) * n_chains, cudaMemcpyDeviceToHost, ctx->stream));
     rc = sl_synchronize(ctx);
     for (void* p : {(void*)d_starts, (void*)d_w}) {
@@ -3822,6 +3929,7 @@ int sl_sequential_imputation_run(sl_ctx* ctx, int32_t iterations, uint64_t seed,
     if ((rc = dev_alloc(ctx, &d_starts, (size_t)C * batch))) return rc;
     if ((rc = dev_alloc(ctx, &d_w, (size_t)C * batch))) return rc;
     if ((rc = dev_alloc(ctx, &d_best, (size_t)C))) return rc;
+    const bool quad = quad_ready(ctx);
     std::vector<double> lowest(C, -DBL_MAX);
     CK(cudaMemcpyAsync(d_best, lowest.data(), sizeof(double) * C, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemsetAsync(scratch, 0, sizeof(uint32_t) * words * C * batch, ctx->stream));
@@ -3839,7 +3947,7 @@ int sl_sequential_imputation_run(sl_ctx* ctx, int32_t iterations, uint64_t seed,
         // pass q of chain c writes graph slot q * C + c of scratch
         { Prof pf_(ctx, SL_KERNEL_LSAMPLER);
         CK(launch_si(P, scratch, 0, C, d_starts, nullptr, 0, seed, (uint64_t)p0, d_w, ctx->d_status, ctx->stream,
-                     ctx->ls_wpb, np, (int64_t)(words * C), ctx->ls_grid)); }
+                     ctx->ls_wpb, np, (int64_t)(words * C), ctx->ls_grid, quad, ctx->sms)); }
         { Prof pf_(ctx, SL_KERNEL_OTHER);
         CK(launch_si_select(scratch, ctx->d_dg, 0, C, words, d_w, d_best, np, ctx->stream)); }
     }

@@ -36,6 +36,12 @@ struct ProblemDev {
     int64_t ls_spill_slots;              // task slots the spill buffer holds per chain
     int32_t ls_spill_chains;             // chains it has slots for
     void* ls_spill;                      // [chains][slots][ls_spill_cells] of the L-sampler's type, or null
+    void* quad_arena;                    // the four-lane L-sampler's rfunctions where eight tasks' do not fit its shared
+                                         // memory: [chains][quad_warps] warps' worth (lsampler_quad_kernel), or null
+    int64_t quad_warps;
+    const uint32_t* quad_prog;           // the operations packed for it (QuadOp, sl_kernels.cu), then each one's first
+    int32_t quad_prog_words;             // word and each meiosis's parent, 16 bits each, in the last quad_tail_words
+    int32_t quad_tail_words;
     int32_t max_child;                   // max children of an op (>= 1)
     int32_t fag_bytes;                   // shared bytes one FAG evaluation needs
     double marker_trans;                 // log(0.5) * 2 * Nnf (descent_graph.cc:22)

@@ -6,8 +6,12 @@
 //                            operation order (bit-exact decisions), T=float
 //                            the batched form.  The form compiled per
 //                            pedigree lives in sl_lsjit.cc.
-//  * si_kernel<T>, si_select_kernel -- sequential imputation passes (one-sided
-//                            L-steps from a start locus) and the best pass.
+//  * lsampler_quad_kernel<T> -- the same with four lanes per task, eight tasks
+//                            per warp: the form that runs unless another is
+//                            asked for or the peel sequence does not suit it.
+//  * si_kernel<T>, si_quad_kernel<T>, si_select_kernel -- sequential imputation
+//                            passes (one-sided L-steps from a start locus), 32
+//                            or 4 lanes each, and the best pass.
 //  * fag_kernel           -- M-sampler likelihoods, thread per (chain, locus):
 //                            founder-allele graph with one meiosis toggled
 //                            (exact mode, and fast mode past the warp form's
@@ -109,7 +113,22 @@ struct Draws {
         uint64_t hi = ((uint64_t)chain << 40) ^ (it << 4) ^ (uint64_t)stage;
         return philox_u01(sd, hi, ((uint64_t)unit << 24) ^ (uint64_t)k);
     }
+    // The same draw rounded down to a float: for a float x, get() < (double)x
+    // exactly when get_rd() < x (no float lies between a draw and the one below
+    // it), without the FP64 units, of which an SM has two.
+    __device__ __forceinline__ float get_rd(int chain_rel, int chain, int64_t unit, int64_t k) const {
+        if (u) return __double2float_rd(u[chain_rel * chain_stride + unit * unit_stride + k]);
+        const uint64_t sd = key ? key[0] : seed, it = key ? key[1] : iter;
+        const uint64_t hi = ((uint64_t)chain << 40) ^ (it << 4) ^ (uint64_t)stage;
+        return __ull2float_rd(sl_philox_bits(sd, hi, ((uint64_t)unit << 24) ^ (uint64_t)k)) * 0x1p-53f;
+    }
 };
+// the draw to compare a probability of type T with
+template <typename T>
+__device__ __forceinline__ T draw_for(const Draws& d, int chain_rel, int chain, int64_t unit, int64_t k) {
+    if constexpr (sizeof(T) == 4) return d.get_rd(chain_rel, chain, unit, k);
+    else return d.get(chain_rel, chain, unit, k);
+}
 
 __global__ void set_key_kernel(uint64_t* key, uint64_t seed, uint64_t iter) {
     key[0] = seed;
@@ -670,6 +689,513 @@ __global__ void __launch_bounds__(128) lsampler_kernel(ProblemDev P, uint32_t* d
     }
 }
 
+// ---------------------------------------------------------------------------
+// L-sampler with four lanes per (chain, locus) task, eight tasks per warp.
+//
+// The steps, products and draws of ls_locus, bit for bit; what differs is how
+// the work lies on the warp.  Lane v of a task's four works out the terms of
+// the peel node's state v, four cells of an rfunction at a time; with most
+// members typed an op has one to four cells, so the eight tasks go through an
+// op together and its description is read once for them, from a packed form of
+// the operations in the block's shared memory (P.quad_prog).  The transmission
+// distributions, which ls_locus works out again for every child, op and pass
+// (four divisions each), take only four values per locus -- a child's indicator
+// at the left and the right neighbour -- and are tabled once per task; likewise
+// the indicator probabilities of the last phase.  A task's shared memory holds
+// a byte per member and the neighbours' columns; the rfunctions, compact as
+// there, lie in shared memory when eight tasks' fit (kQuadSharedArena), else
+// in a global arena that stays in L1 and L2.
+//
+// Bound by issue: 400,000 warp instructions per eight tasks of the 400-member
+// pedigree, 58% of the issue slots with 15 warps on an SM.  The loops stay
+// rolled: unrolled by the compiler, warps at different operations waited for
+// instructions (8 chains of that pedigree 12.7 ms a sweep, rolled 6.4).
+// Measured, a sweep (the fastest of 32, 16 and 8 lanes before): 400 members,
+// 10,000 SNPs, one chain 4.2 -> 2.2 ms, 8 chains 30.1 -> 5.7, 32 chains 123 ->
+// 22.3; 120 members, 2,000 SNPs, one chain 0.86 -> 0.59, 10 chains 2.1 -> 0.71;
+// 30 members, 200 SNPs, one chain 0.23 -> 0.17.
+// ---------------------------------------------------------------------------
+constexpr int kQuadTasks = 8;                       // tasks per warp
+constexpr int kQuadWarps = 8;                       // most warps per block
+constexpr size_t kQuadSharedArena = 20 * 1024;      // most shared bytes per warp with the rfunctions in them
+
+__host__ __device__ __forceinline__ size_t quad_cols_at(const ProblemDev& P) { return al16((size_t)P.N * kQuadTasks); }
+__host__ __device__ __forceinline__ size_t quad_off_at(const ProblemDev& P) {
+    return quad_cols_at(P) + al16((size_t)2 * P.W * 4 * kQuadTasks);
+}
+template <typename T>
+__host__ __device__ __forceinline__ size_t quad_tab_at(const ProblemDev& P) {
+    return quad_off_at(P) + al16((size_t)2 * P.K * kQuadTasks);
+}
+// [32] transmission values and [16] priors per task, then the rfunctions
+template <typename T>
+__host__ __device__ __forceinline__ size_t quad_arena_at(const ProblemDev& P) {
+    return quad_tab_at<T>(P) + 48 * sizeof(T) * kQuadTasks;
+}
+template <typename T>
+__host__ __device__ __forceinline__ size_t quad_arena_bytes(const ProblemDev& P) {
+    return al16((size_t)(P.ls_arena | 1) * sizeof(T) * kQuadTasks);
+}
+template <typename T>
+__host__ __device__ __forceinline__ bool quad_arena_shared(const ProblemDev& P) {
+    return quad_arena_at<T>(P) + quad_arena_bytes<T>(P) <= kQuadSharedArena;
+}
+template <typename T>
+__host__ __device__ __forceinline__ size_t quad_warp_bytes(const ProblemDev& P) {
+    return quad_arena_at<T>(P) + (quad_arena_shared<T>(P) ? quad_arena_bytes<T>(P) : 0);
+}
+// shared bytes of a block's copy of the operations (0: they stay in global memory)
+__host__ __device__ __forceinline__ size_t quad_prog_bytes(const ProblemDev& P) {
+    return P.quad_prog_words <= 8 * 1024 ? al16((size_t)P.quad_prog_words * 4) : 0;
+}
+// bits 2 r and 2 r + 1 of entry m: the r-th state that mask m allows
+__device__ __forceinline__ unsigned quad_states(int m) {
+    unsigned s = 0;
+    int r = 0;
+    for (int v = 0; v < 4; ++v)
+        if ((m >> v) & 1) {
+            s |= (unsigned)v << (2 * r);
+            ++r;
+        }
+    return s;
+}
+
+// One operation of P.quad_prog: word 0 its sizes (below), word 1 the peel node,
+// then the cutset members, two to a word; per previous rfunction its op and
+// cutset size, then its keys' positions (four bits each; the peel node's is c);
+// per child (for a child peel, the peel node itself) its first meiosis, and for
+// a parent peel its position, the other parent's and whether the peel node is
+// its mother.
+struct QuadOp {
+    const uint32_t *cuts, *prevs, *kids;
+    int type, c, n_prev, n_kid, mpos, fpos, peel;
+    __device__ __forceinline__ explicit QuadOp(const uint32_t* w) {
+        const uint32_t h = w[0];
+        peel = (int)w[1];
+        c = h & 15;
+        type = (h >> 4) & 7;
+        n_prev = (h >> 7) & 31;
+        n_kid = (h >> 12) & 31;
+        mpos = (h >> 17) & 15;
+        fpos = (h >> 21) & 15;
+        cuts = w + 2;
+        prevs = cuts + ((c + 1) >> 1);
+        kids = prevs + 2 * n_prev;
+    }
+    __device__ __forceinline__ int cut(int q) const { return (int)(cuts[q >> 1] >> (16 * (q & 1))) & 0xffff; }
+};
+
+// What a task's lanes share: byte arrays [members][8], words [2 W][8], and so on.
+template <typename T>
+struct Quad {
+    const ProblemDev& P;
+    const uint32_t* prog;   // the operations (QuadOp)
+    const uint16_t* at;     // [K] each one's first word
+    const uint16_t* parent; // [2 Nnf] the parent of each meiosis
+    uint8_t* geno;     // bits 0-1 genotype code, bits 2-3 the sampled state, bits 4-7 allowed states
+    uint32_t* cols;    // the left neighbour's words, then the right one's
+    uint16_t* off;     // each op's first cell
+    T* tab;            // [indicators of the two neighbours][parent's state][allele]
+    T* pri;            // [genotype code][state]
+    T* A;              // this task's rfunctions
+    int task, v;
+    __device__ __forceinline__ int mem(int i) const { return geno[i * kQuadTasks + task]; }
+    __device__ __forceinline__ int bits2(int b) const {   // meiosis b's indicators: left, right << 1
+        const int w = b >> 5;
+        return (int)((cols[w * kQuadTasks + task] >> (b & 31)) & 1u) |
+               (int)((cols[(P.W + w) * kQuadTasks + task] >> (b & 31)) & 1u) << 1;
+    }
+    // the probability that a parent in state st passes on `allele` (ls_dist_one's d[2 st + allele])
+    __device__ __forceinline__ T dist(int ind, int st, int allele) const {
+        return tab[(8 * ind + 2 * st + allele) * kQuadTasks + task];
+    }
+    // the op's children's indicators, four bits each in order
+    __device__ __forceinline__ unsigned long long children(const QuadOp& op) const {
+        unsigned long long x = 0;
+#pragma unroll 1
+        for (int c = 0; c < op.n_kid; ++c) {
+            const int b = (int)op.kids[c] & 0xffff;
+            x |= (unsigned long long)(bits2(b) | bits2(b + 1) << 2) << (4 * c);
+        }
+        return x;
+    }
+    // ls_term of NC cells for this lane's state (tv its prior, vbit whether it is
+    // allowed): ext and rk hold each cell's states and ranks, two bits a position.
+    // Every index read is inside its rfunction, whatever the cell.
+    template <int NC>
+    __device__ __forceinline__ void term(const QuadOp& op, unsigned long long ch, const int (&ext)[NC],
+                                         const int (&rk)[NC], int bits, bool vbit, T tv, T (&t)[NC]) const {
+        using Ar = Ls<T>;
+#pragma unroll
+        for (int n = 0; n < NC; ++n) t[n] = tv;
+        if (op.type == CHILD) {
+            const int m = 8 * ((int)ch & 3) + mat_allele(v), p = 8 * ((int)(ch >> 2) & 3) + pat_allele(v);
+#pragma unroll
+            for (int n = 0; n < NC; ++n)
+                t[n] = Ar::mul(t[n], Ar::mul(tab[(m + 2 * digit(ext[n], op.mpos)) * kQuadTasks + task],
+                                             tab[(p + 2 * digit(ext[n], op.fpos)) * kQuadTasks + task]));
+        }
+#pragma unroll 1
+        for (int j = 0; j < op.n_prev; ++j) {
+            const uint32_t w = op.prevs[2 * j];
+            uint32_t keys = op.prevs[2 * j + 1];
+            int idx[NC], sh = 0;
+#pragma unroll
+            for (int n = 0; n < NC; ++n) idx[n] = 0;
+            bool good = true;
+#pragma unroll 1
+            for (int q = (int)w >> 16; q > 0; --q, keys >>= 4) {
+                const int pos = keys & 15, p2 = 2 * pos;
+#pragma unroll
+                for (int n = 0; n < NC; ++n) idx[n] |= ((rk[n] >> p2) & 3) << sh;
+                sh += (bits >> p2) & 3;
+                good &= vbit || pos != op.c;
+            }
+            const T* a = A + off[(w & 0xffff) * kQuadTasks + task];
+#pragma unroll
+            for (int n = 0; n < NC; ++n) t[n] = Ar::mul(t[n], good ? a[idx[n]] : T(0));
+        }
+        if (op.type == PARENT) {
+            T cp[NC];
+#pragma unroll
+            for (int n = 0; n < NC; ++n) cp[n] = T(1);
+#pragma unroll 1
+            for (int c = 0; c < op.n_kid; ++c) {
+                const uint32_t w = op.kids[c];
+                const int ind = (int)(ch >> (4 * c)), kp = 2 * ((w >> 16) & 15), op2 = 2 * ((w >> 20) & 15);
+                const bool mum = (w >> 24) & 1;
+#pragma unroll
+                for (int n = 0; n < NC; ++n) {
+                    const int kt = (ext[n] >> kp) & 3, other = (ext[n] >> op2) & 3;
+                    cp[n] = Ar::mul(cp[n], Ar::mul(dist(ind & 3, mum ? v : other, mat_allele(kt)),
+                                                   dist((ind >> 2) & 3, mum ? other : v, pat_allele(kt))));
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < NC; ++n) t[n] = Ar::mul(t[n], cp[n]);
+        }
+    }
+};
+
+// What the forward pass knows of an op at a task.
+struct QuadCells {
+    unsigned long long perm;   // each member's allowed states by rank (8 bits a member)
+    int bits, three;           // rank bits (2 bits a position, the peel node's last); members with three states
+    int vext, vrank;           // this lane's state and rank in the peel node's position
+    bool vbit;                 // the state is allowed
+};
+
+// The totals of cells first .. first + NC - 1 of an op, on all four lanes of each task.
+template <typename T, int NC>
+__device__ __forceinline__ void quad_cells(const Quad<T>& Q, const QuadOp& op, const QuadCells& x,
+                                           unsigned long long ch, int first, int ncell, T tv, int q0, T (&total)[NC]) {
+    using Ar = Ls<T>;
+    int ext[NC], rk[NC], rem[NC];
+    bool ok[NC];
+#pragma unroll
+    for (int n = 0; n < NC; ++n) {
+        ext[n] = x.vext;
+        rk[n] = x.vrank;
+        rem[n] = first + n;
+        ok[n] = first + n < ncell;
+    }
+#pragma unroll 1
+    for (int q = 0; q < op.c; ++q) {
+        const int b = (x.bits >> (2 * q)) & 3, mask = (1 << b) - 1;
+        const unsigned pq = (unsigned)(x.perm >> (8 * q)) & 255u;
+        const bool three = (x.three >> q) & 1;
+#pragma unroll
+        for (int n = 0; n < NC; ++n) {
+            const int r = rem[n] & mask;
+            rem[n] >>= b;
+            ok[n] &= !(three && r == 3);
+            ext[n] |= (int)((pq >> (2 * r)) & 3u) << (2 * q);
+            rk[n] |= r << (2 * q);
+        }
+    }
+    T t[NC];
+    Q.term(op, ch, ext, rk, x.bits, x.vbit, tv, t);
+#pragma unroll
+    for (int n = 0; n < NC; ++n) {
+        const T tn = ok[n] ? t[n] : T(0);
+        const T t0 = __shfl_sync(FULLMASK, tn, q0), t1 = __shfl_sync(FULLMASK, tn, q0 + 1);
+        const T t2 = __shfl_sync(FULLMASK, tn, q0 + 2), t3 = __shfl_sync(FULLMASK, tn, q0 + 3);
+        total[n] = Ar::add(Ar::add(Ar::add(Ar::add(T(0), t0), t1), t2), t3);
+    }
+}
+
+// ls_locus by four lanes; `live` false: a lane group without a task, which
+// goes along with the warp on a task of another's inputs and writes nothing.
+template <typename T>
+__device__ int quad_locus(Quad<T>& Q, const unsigned* states, uint32_t* colC, int cr, int chain, int l, bool hasL,
+                          bool hasR, bool live, const Draws& draws, int64_t unit, int64_t base, int* status,
+                          double* logroot) {
+    using Ar = Ls<T>;
+    constexpr bool kRescale = sizeof(T) == 4;
+    const ProblemDev& P = Q.P;
+    const int lane = threadIdx.x & 31, q0 = lane & ~3, v = Q.v, task = Q.task;
+    // the locus's inputs: genotypes, neighbours' columns, transmission values, priors
+    {
+        const uint8_t* gsrc = P.geno + (size_t)l * P.N;
+#pragma unroll 8
+        for (int i = v; i < P.N; i += 4) Q.geno[i * kQuadTasks + task] = gsrc[i] & 0xf3;
+        for (int w = v; w < P.W; w += 4) {
+            Q.cols[w * kQuadTasks + task] = hasL ? colC[w - P.W] : 0u;
+            Q.cols[(P.W + w) * kQuadTasks + task] = hasR ? colC[w + P.W] : 0u;
+        }
+    }
+    T th = T(1), an = T(1), th2 = T(1), an2 = T(1);
+    if constexpr (sizeof(T) == 4) {
+        const float* tf = P.c_theta_f + (size_t)chain * (P.M - 1);
+        if (hasL) { th2 = tf[l - 1]; an2 = 1.f - th2; }
+        if (hasR) { th = tf[l]; an = 1.f - th; }
+    } else {
+        const double* td = P.c_theta + (size_t)chain * (P.M - 1);
+        if (hasL) { th2 = td[l - 1]; an2 = DSUB(1.0, td[l - 1]); }
+        if (hasR) { th = td[l]; an = DSUB(1.0, td[l]); }
+    }
+    T pick0;   // lane v: the probability of indicator 0 below a homozygous parent, neighbours' indicators v
+    {
+        T t0 = T(0.5), t1 = T(0.5), p0 = T(1), p1 = T(1);
+        if (hasL) {
+            const bool cross = v & 1;
+            t0 = Ar::mul(t0, cross ? th2 : an2);
+            t1 = Ar::mul(t1, cross ? an2 : th2);
+            p0 = Ar::mul(p0, cross ? th2 : an2);
+            p1 = Ar::mul(p1, cross ? an2 : th2);
+        }
+        if (hasR) {
+            const bool cross = v >> 1;
+            t0 = Ar::mul(t0, cross ? th : an);
+            t1 = Ar::mul(t1, cross ? an : th);
+            p0 = Ar::mul(p0, cross ? th : an);
+            p1 = Ar::mul(p1, cross ? an : th);
+        }
+        const T total = Ar::add(t0, t1), uau = Ar::div(t1, total), uua = Ar::div(t0, total);
+        const T d[8] = {T(1), T(0), T(0), T(1), uau, Ar::sub(T(1), uau), uua, Ar::sub(T(1), uua)};   // UU, AA, AU, UA
+        for (int i = 0; i < 8; ++i) Q.tab[(8 * v + i) * kQuadTasks + task] = d[i];
+        pick0 = Ar::div(p0, Ar::add(p0, p1));
+        for (int i = v; i < 16; i += 4) {
+            if constexpr (sizeof(T) == 4) Q.pri[i * kQuadTasks + task] = (T)P.prior_f[(size_t)l * 16 + i];
+            else Q.pri[i * kQuadTasks + task] = (T)P.prior[(size_t)l * 16 + i];
+        }
+    }
+    __syncwarp();
+    int scale = 0, run = 0;
+    T root = T(0);
+    // forward peel over the valid cells of every rfunction
+#pragma unroll 1
+    for (int k = 0; k < P.K; ++k) {
+        const QuadOp op(Q.prog + Q.at[k]);
+        QuadCells x;
+        x.perm = 0;
+        x.bits = x.three = 0;
+        int B = 0;
+#pragma unroll 1
+        for (int q = 0; q < op.c; ++q) {
+            const int m = Q.mem(op.cut(q)) >> 4, b = rank_bits(m);
+            x.perm |= (unsigned long long)states[m] << (8 * q);
+            x.bits |= b << (2 * q);
+            B += b;
+            x.three |= (__popc(m) == 3) << q;
+        }
+        const int gp = Q.mem(op.peel), mp = gp >> 4;
+        const int ncell = 1 << B;
+        const T tv = Q.pri[(4 * (gp & 3) + v) * kQuadTasks + task];
+        x.vbit = (mp >> v) & 1;
+        x.bits |= rank_bits(mp) << (2 * op.c);
+        x.vrank = x.vbit ? state_rank(mp, v) << (2 * op.c) : 0;
+        x.vext = v << (2 * op.c);
+        const unsigned long long ch = Q.children(op);
+        const int most = __reduce_max_sync(FULLMASK, B);   // the warp's widest task
+        const int ob = run;
+        // all four lanes have each total; up to four cells wait in registers (cell v in lane v) for the scaling
+        T mx = T(0), mine = T(0);
+        if (most < 2) {
+            T t[2];
+            quad_cells<T, 2>(Q, op, x, ch, 0, ncell, tv, q0, t);
+            mx = t[0] > mx ? t[0] : mx;
+            mx = t[1] > mx ? t[1] : mx;
+            mine = v == 0 ? t[0] : t[1];
+        } else {
+#pragma unroll 1
+            for (int cell = 0; cell < 1 << most; cell += 4) {
+                T t[4];
+                quad_cells<T, 4>(Q, op, x, ch, cell, ncell, tv, q0, t);
+#pragma unroll
+                for (int n = 0; n < 4; ++n) mx = t[n] > mx ? t[n] : mx;
+                const T m = v == 0 ? t[0] : v == 1 ? t[1] : v == 2 ? t[2] : t[3];
+                if (cell == 0) mine = m;
+                if (ncell > 4 && cell < ncell) Q.A[ob + cell + v] = m;
+            }
+        }
+        if (k == P.K - 1) root = __shfl_sync(FULLMASK, mine, q0);
+        if (kRescale) {
+            float f = 1.f;
+            if (mx > T(0)) {
+                const int ex = ilogbf((float)mx);
+                scale += ex;
+                f = scalbnf(1.0f, -ex);
+                if (k == P.K - 1) root = (T)((float)root * f);
+            }
+            if (ncell > 4) {
+                if (mx > T(0))
+#pragma unroll 1
+                    for (int cell = v; cell < ncell; cell += 4) Q.A[ob + cell] = (T)((float)Q.A[ob + cell] * f);
+            } else if (v < ncell) {
+                Q.A[ob + v] = mx > T(0) ? (T)((float)mine * f) : mine;
+            }
+        } else if (ncell <= 4 && v < ncell) {
+            Q.A[ob + v] = mine;
+        }
+        if (v == 0) Q.off[k * kQuadTasks + task] = (uint16_t)ob;
+        run += ncell;
+        __syncwarp();
+    }
+    bool fail = false;
+    if (root == T(0)) {
+        if (live && v == 0) set_status(status, ST_ZERO_LIK);
+        fail = true;
+    }
+    if (v == 0 && logroot && !fail) *logroot = log((double)root) + (double)scale * 0.69314718055994530942;
+    // backward sampling of ordered genotypes: lane v draws the uniforms of every fourth operation
+    T draw = T(0);
+#pragma unroll 1
+    for (int j = 0; j < P.K; ++j) {
+        const int k = P.K - 1 - j;
+        const QuadOp op(Q.prog + Q.at[k]);
+        if ((j & 3) == 0 && j + v < P.K && live && !fail) draw = draw_for<T>(draws, cr, chain, unit, base + j + v);
+        int ext[1] = {v << (2 * op.c)}, rk[1] = {0}, bits = 0;
+        bool ok = true;
+#pragma unroll 1
+        for (int q = 0; q < op.c; ++q) {
+            const int g = Q.mem(op.cut(q)), a = (g >> 2) & 3, m = g >> 4;
+            const bool in = (m >> a) & 1;
+            ok &= in;
+            ext[0] |= a << (2 * q);
+            rk[0] |= in ? state_rank(m, a) << (2 * q) : 0;
+            bits |= rank_bits(m) << (2 * q);
+        }
+        const int gp = Q.mem(op.peel), mp = gp >> 4;
+        const T tv = Q.pri[(4 * (gp & 3) + v) * kQuadTasks + task];
+        const bool vbit = (mp >> v) & 1;
+        rk[0] |= vbit ? state_rank(mp, v) << (2 * op.c) : 0;
+        bits |= rank_bits(mp) << (2 * op.c);
+        T pt[1];
+        Q.term(op, Q.children(op), ext, rk, bits, vbit, tv, pt);
+        const T pv = ok ? pt[0] : T(0);
+        const T r = __shfl_sync(FULLMASK, draw, q0 + (j & 3));
+        const T p0 = __shfl_sync(FULLMASK, pv, q0), p1 = __shfl_sync(FULLMASK, pv, q0 + 1);
+        const T p2 = __shfl_sync(FULLMASK, pv, q0 + 2), p3 = __shfl_sync(FULLMASK, pv, q0 + 3);
+        const T tot = Ar::add(Ar::add(Ar::add(p0, p1), p2), p3);
+        // lane v divides its own term; the four quotients are added up in order
+        const T d = tot != T(0) ? Ar::div(pv, tot) : pv;
+        const T d0 = __shfl_sync(FULLMASK, d, q0), d1 = __shfl_sync(FULLMASK, d, q0 + 1);
+        const T d2 = __shfl_sync(FULLMASK, d, q0 + 2), d3 = __shfl_sync(FULLMASK, d, q0 + 3);
+        const T a0 = Ar::add(T(0), d0), a1 = Ar::add(a0, d1), a2 = Ar::add(a1, d2), a3 = Ar::add(a2, d3);
+        int pick;
+        if (r < a0) pick = 0;
+        else if (r < a1) pick = 1;
+        else if (r < a2) pick = 2;
+        else if (r < a3) pick = 3;
+        else pick = d3 != T(0) ? 3 : d2 != T(0) ? 2 : d1 != T(0) ? 1 : 0;
+        if (v == 0) Q.geno[op.peel * kQuadTasks + task] = (uint8_t)((gp & 0xf3) | pick << 2);
+        __syncwarp();
+    }
+    // meiosis indicators in person order, maternal first, four at a time; a
+    // draw is consumed only below a homozygous parent
+    int64_t cursor = base + P.K;
+    const int nb = 2 * P.Nnf;
+#pragma unroll 1
+    for (int w = 0; w < P.W; ++w) {
+        uint32_t word = 0;
+#pragma unroll 1
+        for (int h = 0; h < 32; h += 4) {
+            const int b = 32 * w + h + v;
+            if (32 * w + h >= nb) break;   // the same for the whole warp
+            int mi = 0, need = 0, ind = 0;
+            if (b < nb) {
+                const int i = P.F + (b >> 1), par = b & 1;
+                const int tr = (Q.mem(i) >> 2) & 3;
+                const int ptr = (Q.mem(Q.parent[b]) >> 2) & 3;
+                const int allele = par == 0 ? ((tr == UU || tr == UA) ? 0 : 1) : ((tr == UU || tr == AU) ? 0 : 1);
+                if (ptr == UA || ptr == AU) mi = (allele == 0) == (ptr == UA) ? 0 : 1;
+                else {
+                    need = 1;
+                    ind = Q.bits2(b);
+                }
+            }
+            const unsigned nmask = (__ballot_sync(FULLMASK, need) >> q0) & 15u;
+            const T p = __shfl_sync(FULLMASK, pick0, q0 + ind);
+            if (need && live && !fail) {
+                const T r = draw_for<T>(draws, cr, chain, unit, cursor + __popc(nmask & ((1u << v) - 1u)));
+                mi = r < p ? 0 : 1;
+            }
+            cursor += __popc(nmask);
+            word |= ((__ballot_sync(FULLMASK, mi != 0) >> q0) & 15u) << h;
+        }
+        if (v == 0 && live && !fail) colC[w] = word;   // bits past 2 Nnf stay zero
+    }
+    __syncwarp();
+    return fail ? -1 : (int)(cursor - base);
+}
+
+// A warp's Quad over its shared memory; arena: its part of the global one.
+template <typename T>
+__device__ __forceinline__ Quad<T> quad_bind(const ProblemDev& P, const uint32_t* prog, unsigned char* wsm, T* arena) {
+    const int lane = threadIdx.x & 31, task = lane >> 2;
+    T* rf = quad_arena_shared<T>(P) ? (T*)(wsm + quad_arena_at<T>(P)) : arena;
+    T* tab = (T*)(wsm + quad_tab_at<T>(P));
+    const uint16_t* at = (const uint16_t*)(prog + P.quad_prog_words - P.quad_tail_words);
+    return Quad<T>{P, prog, at, at + P.K, wsm, (uint32_t*)(wsm + quad_cols_at(P)), (uint16_t*)(wsm + quad_off_at(P)), tab,
+                   tab + 32 * kQuadTasks, rf + (size_t)task * (P.ls_arena | 1), task, lane & 3};
+}
+
+// The block's copies of the operations and of quad_states.
+__device__ __forceinline__ const uint32_t* quad_stage(const ProblemDev& P, unsigned char* smem, unsigned* states) {
+    const uint32_t* prog = P.quad_prog;
+    if (quad_prog_bytes(P)) {
+        uint32_t* sp = (uint32_t*)smem;
+        for (int i = threadIdx.x; i < P.quad_prog_words; i += blockDim.x) sp[i] = prog[i];
+        prog = sp;
+    }
+    if (threadIdx.x < 16) states[threadIdx.x] = quad_states(threadIdx.x);
+    __syncthreads();
+    return prog;
+}
+
+// This launch's warp w of chains from `first` on: its part of the global arena
+// (null: the rfunctions are in shared memory).
+template <typename T>
+__device__ __forceinline__ T* quad_arena_slice(const ProblemDev& P, int first, int64_t w) {
+    if (quad_arena_shared<T>(P)) return nullptr;
+    return (T*)P.quad_arena + ((size_t)first * P.quad_warps + w) * (quad_arena_bytes<T>(P) / sizeof(T));
+}
+
+template <typename T>
+__global__ void __launch_bounds__(32 * kQuadWarps) lsampler_quad_kernel(ProblemDev P, uint32_t* dg, int first,
+                                                                        int nchain, const int32_t* loci, int nloci,
+                                                                        Draws draws, const uint8_t* sel, int want,
+                                                                        int* status) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ unsigned states[16];
+    const uint32_t* prog = quad_stage(P, smem, states);
+    const int warp = threadIdx.x >> 5;
+    const int wpb = blockDim.x >> 5;
+    const int64_t gw = (int64_t)blockIdx.x * wpb + warp, nw = (int64_t)gridDim.x * wpb;
+    Quad<T> Q = quad_bind<T>(P, prog, smem + quad_prog_bytes(P) + warp * quad_warp_bytes<T>(P),
+                             quad_arena_slice<T>(P, first, gw));
+    const int64_t ntask = (int64_t)nchain * nloci;
+    for (int64_t g = gw; g * kQuadTasks < ntask; g += nw) {
+        const int64_t t = min(g * kQuadTasks + Q.task, ntask - 1);
+        const int cr = (int)(t / nloci), l = loci[t % nloci];
+        const bool live = g * kQuadTasks + Q.task < ntask && !(sel && sel[cr] != want);
+        if (!__any_sync(FULLMASK, live)) continue;
+        uint32_t* colC = dg + ((size_t)(first + cr) * P.M + l) * P.W;
+        quad_locus<T>(Q, states, colC, cr, first + cr, l, l > 0, l < P.M - 1, live, draws, l, 0, status, nullptr);
+    }
+}
+
 // Sequential imputation (LocusSampler::start_from, locus_sampler2.cc:214-241),
 // one warp per chain: the start locus with neither neighbour, then leftwards
 // with the right neighbour only, then rightwards with the left neighbour only;
@@ -719,6 +1245,49 @@ __global__ void __launch_bounds__(128) si_kernel(ProblemDev P, uint32_t* dg, int
             w += __shfl_sync(FULLMASK, lr, 0);
         }
         if (lane == 0) weights[t] = ok ? w : -DBL_MAX;
+        __syncwarp();
+    }
+}
+
+// The same by four lanes per pass (quad_locus), eight passes a warp; a pass
+// that met a locus of likelihood 0 goes along with its warp and writes nothing
+// more.  1,000 passes of 301 loci of the 120-member pedigree: 133 -> 74 ms, bound
+// by one pass's chain of loci (125 warps on the whole GPU).
+template <typename T>
+__global__ void __launch_bounds__(32 * kQuadWarps) si_quad_kernel(ProblemDev P, uint32_t* dg, int first, int nchain,
+                                                                  const int32_t* starts, Draws draws, int64_t unit,
+                                                                  double* weights, int* status, int npass,
+                                                                  int64_t pass_stride) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ unsigned states[16];
+    const uint32_t* prog = quad_stage(P, smem, states);
+    const int warp = threadIdx.x >> 5, wpb = blockDim.x >> 5, M = P.M;
+    const int64_t gw = (int64_t)blockIdx.x * wpb + warp, nw = (int64_t)gridDim.x * wpb;
+    Quad<T> Q = quad_bind<T>(P, prog, smem + quad_prog_bytes(P) + warp * quad_warp_bytes<T>(P),
+                             quad_arena_slice<T>(P, first, gw));
+    const int64_t ntask = (int64_t)nchain * npass;
+    for (int64_t g = gw; g * kQuadTasks < ntask; g += nw) {
+        const int64_t t = min(g * kQuadTasks + Q.task, ntask - 1);
+        const int cr = (int)(t % nchain), q = (int)(t / nchain), chain = first + cr, start = starts[t];
+        const bool mine = g * kQuadTasks + Q.task < ntask;
+        uint32_t* graph = dg + (size_t)q * pass_stride + (size_t)chain * M * P.W;
+        Draws dq = draws;
+        dq.iter = draws.iter + (uint64_t)q;
+        int64_t base = 0;
+        double w = 0.0;
+        bool ok = mine;
+        for (int k = 0; k < M && __any_sync(FULLMASK, ok); ++k) {
+            const int l = k == 0 ? start : (k <= start ? start - k : k);
+            const bool hasL = k > start && l > 0;
+            const bool hasR = k > 0 && k <= start && l < M - 1;
+            double lr = 0.0;
+            const int used = quad_locus<T>(Q, states, graph + (size_t)l * P.W, cr, chain, l, hasL, hasR, ok, dq, unit,
+                                           base, status, &lr);
+            if (used < 0) ok = false;
+            base += used;
+            w += lr;
+        }
+        if (mine && Q.v == 0) weights[t] = ok ? w : -DBL_MAX;
         __syncwarp();
     }
 }
@@ -3607,12 +4176,52 @@ int lsampler_resident_tasks(const ProblemDev& P, int wpb) {
     return P.ls_fast ? ls_resident_t<float>(P, wpb) : ls_resident_t<double>(P, wpb);
 }
 
-// lanes = 32, 16 or 8 lanes per (chain, locus) task; all draw the same graphs.
+// Bytes of global arena a warp of the four-lane kernel needs (0: none, its
+// rfunctions are in shared memory), and its shared bytes per block.
+size_t quad_arena_per_warp(const ProblemDev& P) {
+    if (P.ls_fast) return quad_arena_shared<float>(P) ? 0 : quad_arena_bytes<float>(P);
+    return quad_arena_shared<double>(P) ? 0 : quad_arena_bytes<double>(P);
+}
+size_t quad_block_bytes(const ProblemDev& P, int warps) {
+    return quad_prog_bytes(P) + warps * (P.ls_fast ? quad_warp_bytes<float>(P) : quad_warp_bytes<double>(P));
+}
+
+// Warps per block of the four-lane kernel: one block of as many as the SM's
+// share of the warps that `load` chains' half-sweeps are, up to 8 and to what
+// fits -- few warps are spread over the SMs, many share their block's copy of
+// the operations (400 members, a sweep of 8 chains: 6.4 ms with 4 warps a block,
+// 5.7 with 8).
+static int quad_warps_per_block(const ProblemDev& P, int64_t load, int nloci, int sms) {
+    const int64_t warps = load * ((nloci + kQuadTasks - 1) / kQuadTasks);
+    int w = (int)std::max<int64_t>(1, std::min<int64_t>(kQuadWarps, (warps + sms - 1) / sms));
+    while (w > 1 && quad_block_bytes(P, w) > 110 * 1024) --w;   // two blocks to an SM
+    return w;
+}
+
+template <typename T>
+static cudaError_t launch_quad(const ProblemDev& P, uint32_t* dg, int first, int nchain, const int32_t* loci, int nloci,
+                               const Draws& d, const uint8_t* sel, int want, int* status, cudaStream_t s, int wpb) {
+    const size_t smem = quad_block_bytes(P, wpb);
+    cudaError_t e = ensure_smem((const void*)lsampler_quad_kernel<T>, smem);
+    if (e != cudaSuccess) return e;
+    const int per = kQuadTasks * wpb;
+    int64_t grid = ((int64_t)nchain * nloci + per - 1) / per;
+    if (quad_arena_per_warp(P)) grid = std::min(grid, nchain * (P.quad_warps / wpb));   // slots of the arena
+    lsampler_quad_kernel<T><<<(int)grid, 32 * wpb, smem, s>>>(P, dg, first, nchain, loci, nloci, d, sel, want, status);
+    return cudaGetLastError();
+}
+
+// lanes = 32, 16, 8 or 4 lanes per (chain, locus) task; all draw the same graphs.
 cudaError_t launch_lsampler(const ProblemDev& P, uint32_t* dg, int first, int nchain, const int32_t* loci, int nloci,
                             const double* u, int64_t ucs, int64_t uls, uint64_t seed, uint64_t iter,
                             const uint8_t* sel, int want, int* status, cudaStream_t s, int grid_cap, int wpb,
-                            const uint64_t* key, int lanes) {
+                            const uint64_t* key, int lanes, int load, int sms) {
     Draws d{u, ucs, uls, seed, iter, 1, key};
+    if (lanes == 4) {
+        const int w4 = quad_warps_per_block(P, std::max(load, nchain), nloci, sms);
+        if (P.ls_fast) return launch_quad<float>(P, dg, first, nchain, loci, nloci, d, sel, want, status, s, w4);
+        return launch_quad<double>(P, dg, first, nchain, loci, nloci, d, sel, want, status, s, w4);
+    }
     if (lanes == 8) {
         // four tasks per warp: a quarter of the warps per block keeps the block's shared memory
         const int w8 = wpb > 3 ? wpb / 4 : 1;
@@ -3655,9 +4264,32 @@ __global__ void si_select_kernel(const uint32_t* scratch, uint32_t* dg, int firs
     }
 }
 
+template <typename T>
+static cudaError_t launch_si_quad(const ProblemDev& P, uint32_t* dg, int first, int nchain, const int32_t* starts,
+                                  const Draws& d, double* weights, int* status, cudaStream_t s, int npass,
+                                  int64_t pass_stride, int sms) {
+    const int64_t ntask = (int64_t)nchain * npass;
+    const int wpb = quad_warps_per_block(P, 1, (int)ntask, sms), per = kQuadTasks * wpb;
+    const size_t smem = quad_block_bytes(P, wpb);
+    cudaError_t e = ensure_smem((const void*)si_quad_kernel<T>, smem);
+    if (e != cudaSuccess) return e;
+    int64_t grid = (ntask + per - 1) / per;
+    if (quad_arena_per_warp(P)) grid = std::min(grid, nchain * (P.quad_warps / wpb));   // slots of the arena
+    si_quad_kernel<T><<<(int)grid, 32 * wpb, smem, s>>>(P, dg, first, nchain, starts, d, 0, weights, status, npass,
+                                                        pass_stride);
+    return cudaGetLastError();
+}
+
+// quad: by four lanes per pass (P.quad_prog set, its arena there)
 cudaError_t launch_si(const ProblemDev& P, uint32_t* dg, int first, int nchain, const int32_t* starts,
                       const double* u, int64_t ucs, uint64_t seed, uint64_t pass, double* weights, int* status,
-                      cudaStream_t s, int wpb, int npass, int64_t pass_stride, int grid_cap) {
+                      cudaStream_t s, int wpb, int npass, int64_t pass_stride, int grid_cap, bool quad, int sms) {
+    if (quad) {
+        const Draws dr{u, ucs, 0, seed, pass, 5, nullptr};
+        if (P.ls_fast)
+            return launch_si_quad<float>(P, dg, first, nchain, starts, dr, weights, status, s, npass, pass_stride, sms);
+        return launch_si_quad<double>(P, dg, first, nchain, starts, dr, weights, status, s, npass, pass_stride, sms);
+    }
     const size_t smem = ls_tables_bytes(P) + wpb * lsampler_smem_per_warp(P);
     {
         cudaError_t e = ensure_smem(P.ls_fast ? (const void*)si_kernel<float> : (const void*)si_kernel<double>, smem);

@@ -5,8 +5,9 @@
 // run time, so every kernel draws the same stream.
 #pragma once
 
-__device__ __forceinline__ double sl_philox_u01(unsigned long long key, unsigned long long c_hi,
-                                                unsigned long long c_lo) {
+// a draw's 53 bits
+__device__ __forceinline__ unsigned long long sl_philox_bits(unsigned long long key, unsigned long long c_hi,
+                                                             unsigned long long c_lo) {
     unsigned int c0 = (unsigned int)c_lo, c1 = (unsigned int)(c_lo >> 32);
     unsigned int c2 = (unsigned int)c_hi, c3 = (unsigned int)(c_hi >> 32);
     unsigned int k0 = (unsigned int)key, k1 = (unsigned int)(key >> 32);
@@ -24,5 +25,10 @@ __device__ __forceinline__ double sl_philox_u01(unsigned long long key, unsigned
         k1 += 0xBB67AE85u;
     }
     const unsigned long long hi = c0 >> 5, lo = c1 >> 6;
-    return (double)(hi * 67108864ull + lo) * (1.0 / 9007199254740992.0);
+    return hi * 67108864ull + lo;
+}
+
+__device__ __forceinline__ double sl_philox_u01(unsigned long long key, unsigned long long c_hi,
+                                                unsigned long long c_lo) {
+    return (double)sl_philox_bits(key, c_hi, c_lo) * (1.0 / 9007199254740992.0);
 }
