@@ -309,16 +309,17 @@ int sl_profile_read(sl_ctx* ctx, int32_t kernel, double* total_ms, int64_t* laun
  *    person.cc:224-299, filled while parsing, pedigree_parser.cc:157);
  *  - log P(T), the trait peel without a descent graph (Peeler::calc_trait_prob,
  *    peeler.cc:65-73);
- *  - what the genotypes alone say about toggling meiosis m (2 (person - F) +
- *    parent) at locus l of a legal descent graph, [2 (N - F)][M]: bit 0 set, the
- *    founder-allele-graph likelihood stays as it is; bit 1 set, it becomes
+ *  - what the genotypes, and the near meioses of a legal descent graph (dg,
+ *    int32 reference layout; NULL: the genotypes alone), say about toggling
+ *    meiosis m (2 (person - F) + parent) at locus l, [2 (N - F)][M]: bit 0 set,
+ *    the founder-allele-graph likelihood stays as it is; bit 1 set, it becomes
  *    zero; neither, the fast M-sampler evaluates it (no counterpart in the
  *    reference, which evaluates every one, meiosis_sampler.cc:123-134).
  */
 int sl_problem_legal_masks(const sl_problem_desc* problem, uint8_t* out);
 int sl_problem_trait_priors(const sl_problem_desc* problem, double* out);
 int sl_problem_trait_prob(const sl_problem_desc* problem, double* out);
-int sl_problem_meiosis_flips(const sl_problem_desc* problem, uint8_t* out);
+int sl_problem_meiosis_flips(const sl_problem_desc* problem, const int32_t* dg, uint8_t* out);
 
 /* The batched LOD form's compiled trait-peel program (its construction is host
  * work), evaluated on the host in FP64 for one descent graph (int32 reference

@@ -62,7 +62,7 @@ def build(verbose: bool = False, force: bool = False) -> str:
     os.makedirs(OUT, exist_ok=True)
     philox = os.path.join(CSRC, "sl_philox.cuh")
     hdrs = [os.path.join(CSRC, "sl_internal.h"), os.path.join(CSRC, "sl_jit.h"), os.path.join(CSRC, "sl_lsjit.h"),
-            os.path.join(CSRC, "sl_adjjit.h"), philox, os.path.join(os.path.dirname(HERE), "include", "swiftlink_gb300.h")]
+            os.path.join(CSRC, "sl_adjjit.h"), os.path.join(CSRC, "sl_flips.h"), philox, os.path.join(os.path.dirname(HERE), "include", "swiftlink_gb300.h")]
     # the Philox source as a C++ string literal, for the run-time compiled kernels
     inc = os.path.join(OUT, "sl_philox_src.inc")
     if force or _stale(inc, [philox]):

@@ -24,6 +24,7 @@
 
 #include "../../include/swiftlink_gb300.h"
 #include "sl_adjjit.h"
+#include "sl_flips.h"
 #include "sl_internal.h"
 #include "sl_jit.h"
 #include "sl_lsjit.h"
@@ -789,6 +790,82 @@ static bool pack_quad_ops(const sl_problem_desc* d, const std::vector<OpDev>& op
     return true;
 }
 
+// The two bits of every member's genotype codes, a bit per locus: [N][2][words].
+static std::vector<uint32_t> genotype_planes(int N, int M, const std::vector<uint8_t>& geno, int words) {
+    std::vector<uint32_t> out((size_t)N * 2 * words, 0), c0(N), c1(N);
+    for (int l0 = 0; l0 < M; l0 += 32) {   // a word of every member's planes at a time
+        std::fill(c0.begin(), c0.end(), 0u);
+        std::fill(c1.begin(), c1.end(), 0u);
+        for (int l = l0; l < std::min(M, l0 + 32); ++l) {
+            const uint8_t* row = geno.data() + (size_t)l * N;
+            for (int i = 0; i < N; ++i) {
+                c0[i] |= (uint32_t)(row[i] & 1) << (l - l0);
+                c1[i] |= (uint32_t)((row[i] >> 1) & 1) << (l - l0);
+            }
+        }
+        for (int i = 0; i < N; ++i) {
+            out[(size_t)2 * i * words + (l0 >> 5)] = c0[i];
+            out[(size_t)(2 * i + 1) * words + (l0 >> 5)] = c1[i];
+        }
+    }
+    return out;
+}
+
+// Every meiosis's relatives (kRelatives in sl_internal.h).
+static std::vector<uint32_t> meiosis_relatives(const sl_problem_desc* d) {
+    const int N = d->n_members, F = d->n_founders;
+    std::vector<std::vector<int>> kids(N);
+    for (int i = F; i < N; ++i) {
+        kids[d->mother[i]].push_back(i);
+        if (d->father[i] != d->mother[i]) kids[d->father[i]].push_back(i);
+    }
+    std::vector<uint32_t> out((size_t)2 * (N - F) * kRelatives, kNoRelative);
+    std::vector<char> under(N);
+    std::vector<int> stack;
+    for (int i = F; i < N; ++i) {
+        if (d->mother[i] == d->father[i]) continue;
+        std::fill(under.begin(), under.end(), 0);
+        under[i] = 1;
+        stack.assign(1, i);
+        while (!stack.empty()) {
+            const int x = stack.back();
+            stack.pop_back();
+            for (int k : kids[x])
+                if (!under[k]) {
+                    under[k] = 1;
+                    stack.push_back(k);
+                }
+        }
+        for (int side = 0; side < 2; ++side) {
+            uint32_t* e = out.data() + (size_t)(2 * (i - F) + side) * kRelatives;
+            const int p = side == 0 ? d->mother[i] : d->father[i], o = side == 0 ? d->father[i] : d->mother[i];
+            e[0] = (uint32_t)i;
+            e[1] = (uint32_t)p;
+            e[2] = (uint32_t)o;
+            if (p >= F) {
+                e[3] = (uint32_t)d->mother[p];
+                e[4] = (uint32_t)d->father[p];
+            }
+            if (o >= F) {
+                e[5] = (uint32_t)d->mother[o];
+                e[6] = (uint32_t)d->father[o];
+            }
+            int n = 7;
+            auto add = [&](int k, uint32_t of) {
+                if (n >= kRelatives || d->mother[k] == d->father[k]) return;
+                const uint32_t male_p = d->father[k] == p, male_o = d->father[k] == o, male_i = d->father[k] == i;
+                e[n++] = (uint32_t)k | of | male_p << 20 | male_o << 21 | male_i << 22;
+            };
+            for (int k : kids[p])
+                if (!under[k]) add(k, kRelOfP | (d->mother[k] == o || d->father[k] == o ? kRelOfO : 0u));
+            for (int k : kids[i]) add(k, kRelOfI);
+            for (int k : kids[o])
+                if (!under[k] && d->mother[k] != p && d->father[k] != p) add(k, kRelOfO);
+        }
+    }
+    return out;
+}
+
 // What a locus's genotypes alone say about toggling a meiosis there
 // (ProblemDev::mflip; the M-sweep evaluates the founder-allele graph only
 // where neither mask holds).  Toggling meiosis (i, p) -- the allele that i has
@@ -807,32 +884,19 @@ static bool pack_quad_ops(const sl_problem_desc* d, const std::vector<OpDev>& op
 // Both hold when the graph as it is is legal; the sweep evaluates the rest.
 // planes: [N][words] bits over the loci.
 static std::vector<uint32_t> meiosis_flips(const sl_problem_desc* d, const std::vector<uint8_t>& geno, int words) {
-    const int N = d->n_members, F = d->n_founders, M = d->n_markers;
+    const int N = d->n_members, F = d->n_founders;
     const size_t W = words;
-    std::vector<uint32_t> hom_a(N * W, 0), hom_b(N * W, 0), het(N * W, 0), below(N * W, 0);
+    std::vector<uint32_t> hom_a(N * W), hom_b(N * W), het(N * W), below(N * W);
     {
-        std::vector<uint32_t> a(N), b(N), h(N);   // a word of every member's planes at a time
-        for (int l0 = 0; l0 < M; l0 += 32) {
-            std::fill(a.begin(), a.end(), 0u);
-            std::fill(b.begin(), b.end(), 0u);
-            std::fill(h.begin(), h.end(), 0u);
-            for (int l = l0; l < std::min(M, l0 + 32); ++l) {
-                const uint8_t* row = geno.data() + (size_t)l * N;
-                for (int i = 0; i < N; ++i) {
-                    const uint32_t g = row[i] & 3u;
-                    a[i] |= (uint32_t)(g == G_HOMOZ_A) << (l - l0);
-                    b[i] |= (uint32_t)(g == G_HOMOZ_B) << (l - l0);
-                    h[i] |= (uint32_t)(g == G_HETERO) << (l - l0);
-                }
+        const std::vector<uint32_t> g = genotype_planes(N, d->n_markers, geno, words);
+        for (int i = 0; i < N; ++i)
+            for (size_t w = 0; w < W; ++w) {
+                const uint32_t c0 = g[2 * i * W + w], c1 = g[(2 * i + 1) * W + w];
+                hom_a[i * W + w] = c1 & ~c0;
+                hom_b[i * W + w] = c1 & c0;
+                het[i * W + w] = c0 & ~c1;
+                below[i * W + w] = c0 | c1;   // i typed; its descendants are added next
             }
-            for (int i = 0; i < N; ++i) {
-                const size_t at = i * W + (l0 >> 5);
-                hom_a[at] = a[i];
-                hom_b[at] = b[i];
-                het[at] = h[i];
-                below[at] = a[i] | b[i] | h[i];   // i typed; its descendants are added next
-            }
-        }
     }
     std::vector<std::vector<int>> kids(N);
     for (int i = F; i < N; ++i) {
@@ -1686,6 +1750,10 @@ int sl_create(const sl_problem_desc* d, const sl_options* opt, sl_ctx** out) {
     if (P.ls_fast) {
         const std::vector<uint32_t> mf = meiosis_flips(d, geno, P.mflip_words);
         if ((rc = upload(ctx, (uint32_t**)&P.mflip, mf.data(), mf.size()))) return bail(rc);
+        const std::vector<uint32_t> gp = genotype_planes(N, M, geno, P.mflip_words);
+        if ((rc = upload(ctx, (uint32_t**)&P.gplane, gp.data(), gp.size()))) return bail(rc);
+        const std::vector<uint32_t> mr = meiosis_relatives(d);
+        if ((rc = upload(ctx, (uint32_t**)&P.mrel, mr.data(), mr.size()))) return bail(rc);
     }
     if ((rc = upload(ctx, (uint8_t**)&P.typed, typed.data(), N))) return bail(rc);
     if ((rc = upload(ctx, (double**)&P.prior, ctx->prior_table.data(), ctx->prior_table.size()))) return bail(rc);
@@ -2300,20 +2368,37 @@ int sl_problem_legal_masks(const sl_problem_desc* d, uint8_t* out) {
     return SL_OK;
 }
 
-int sl_problem_meiosis_flips(const sl_problem_desc* d, uint8_t* out) {
+int sl_problem_meiosis_flips(const sl_problem_desc* d, const int32_t* dg, uint8_t* out) {
     sl_ctx* ctx = nullptr;
     int rc = check_desc(d);
     if (rc) return rc;
     if (!out) return fail(ctx, SL_EINVAL, "null argument");
-    const int N = d->n_members, M = d->n_markers, nm = 2 * (N - d->n_founders), words = (M + 31) / 32;
+    const int N = d->n_members, F = d->n_founders, M = d->n_markers, nm = 2 * (N - F), words = (M + 31) / 32;
     std::vector<uint8_t> geno((size_t)M * N);
     for (size_t i = 0; i < geno.size(); ++i) geno[i] = d->typed[i % N] ? d->genotypes[i] & 3 : 0;
-    const std::vector<uint32_t> mf = meiosis_flips(d, geno, words);
-    for (int m = 0; m < nm; ++m)
-        for (int l = 0; l < M; ++l) {
-            const uint32_t* w = mf.data() + (size_t)m * 2 * words + (l >> 5);
-            out[(size_t)m * M + l] = (uint8_t)((w[0] >> (l & 31) & 1) | (w[words] >> (l & 31) & 1) << 1);
+    const std::vector<uint32_t> mf = meiosis_flips(d, geno, words), gp = genotype_planes(N, M, geno, words);
+    const std::vector<uint32_t> mr = meiosis_relatives(d);
+    for (int w = 0; w < words; ++w) {
+        const int n = std::min(32, M - 32 * w);
+        std::vector<uint32_t> bits(nm, 0u);   // every meiosis's indicators at the word's loci
+        if (dg)
+            for (int l = 0; l < n; ++l)
+                for (int m = 0; m < nm; ++m)
+                    bits[m] |= (uint32_t)(dg[(size_t)(32 * w + l) * 2 * N + 2 * F + m] & 1) << l;
+        for (int m = 0; m < nm; ++m) {
+            uint32_t same = mf[(size_t)m * 2 * words + w], never = mf[((size_t)m * 2 + 1) * words + w];
+            if (dg) {
+                auto entry = [&](int r) { return mr[(size_t)m * kRelatives + r]; };
+                auto code = [&](int r, int k) {
+                    return entry(r) == kNoRelative ? 0u : gp[((size_t)(entry(r) & 0xffffu) * 2 + k) * words + w];
+                };
+                relatives_rule(m, F, bits[m], entry, [&](int r) { return code(r, 0); },
+                               [&](int r) { return code(r, 1); }, [&](int b) { return bits[b]; }, &same, &never);
+            }
+            for (int l = 0; l < n; ++l)
+                out[(size_t)m * M + 32 * w + l] = (uint8_t)((same >> l & 1) | (never >> l & 1) << 1);
         }
+    }
     return SL_OK;
 }
 

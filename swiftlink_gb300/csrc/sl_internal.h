@@ -25,6 +25,15 @@ struct OpDev {
     int32_t prev_ops_at; // opdata offset: the op index of each previous rfunction, in prev_at's order
 };
 
+// The relatives of meiosis (i, p), o being i's other parent: i, p, o, p's
+// mother and father, o's mother and father (kNoRelative where there is none),
+// then children of p or o outside i's descendants and children of i, as many
+// as there is room for, up to the first kNoRelative.  A child's entry says
+// whose it is and, in bits 20-22, which parent (0 mother) p, o and i are to it.
+constexpr int kRelatives = 32;
+constexpr uint32_t kNoRelative = 0xffffffffu;
+constexpr uint32_t kRelOfP = 1u << 16, kRelOfO = 1u << 17, kRelOfI = 1u << 18;
+
 // Everything a kernel needs about one problem; passed by value.
 struct ProblemDev {
     int32_t N, F, M, K, n_lod, Nnf, W;   // W = 32-bit words per descent-graph column
@@ -59,6 +68,8 @@ struct ProblemDev {
                                          // it zero, whatever the rest of a legal graph (meiosis_flips, sl_host.cc); null
                                          // in the exact mode
     int32_t mflip_words;                 // ceil(M / 32)
+    const uint32_t* gplane;              // [N][2][mflip_words]: the two bits of a member's genotype codes, a bit per locus
+    const uint32_t* mrel;                // [2 Nnf meioses][kRelatives]: the meiosis's relatives (flips_by_relatives)
     const double* prior;                 // [M][4 genotype codes][4 states]
     const double* theta;                 // [M-1]
     const double* partial;               // [M-1]

@@ -52,6 +52,7 @@
 #include <mutex>
 #include <utility>
 
+#include "sl_flips.h"
 #include "sl_internal.h"
 #include "sl_philox.cuh"
 
@@ -1855,6 +1856,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // whatever other lanes do meanwhile.
 __device__ __forceinline__ int pf_find(volatile int* L, int x, int& parity) {
     int p = 0, y = x;
+#pragma unroll 1
     for (int it = 0; it < 8192; ++it) {
         const int v = L[y];
         const int up = v >> 1;
@@ -1940,17 +1942,21 @@ __device__ __forceinline__ float fagw_like(const ProblemDev& P, const FagwTables
     const uint32_t cw = wreg && gl < P.W ? col[gl] : 0u;
     const int t0 = P.typ_off[lc], ntyp = P.typ_cnt[lc], nhet = P.typ_nhet[lc];
     const float2 lfreq = P.c_lfreq[(size_t)chain * M + lc];
+#pragma unroll 1
     for (int q = gl; q < (ntyp + 7) >> 3; q += G) cp_async16(typ + 8 * q, P.typ_ent + t0 + 8 * q);
     cp_async_commit();
     // 1. founder alleles, one generation level at a time
+#pragma unroll 1
     for (int q = gl; q < s_off[1]; q += G) {
         const int pid = (int)s_lvl[q].x;
         e[2 * pid] = (E)(2 * pid);
         e[2 * pid + 1] = (E)(2 * pid + 1);
     }
     __syncwarp();
+#pragma unroll 1
     for (int k = 1; k < P.n_lvl; ++k) {
         // every lane takes part in the shuffles, members or not
+#pragma unroll 1
         for (int q0 = s_off[k]; q0 < s_off[k + 1]; q0 += G) {
             const int q = q0 + gl;
             const bool act = q < s_off[k + 1];
@@ -1970,6 +1976,7 @@ __device__ __forceinline__ float fagw_like(const ProblemDev& P, const FagwTables
     // heterozygotes in the list) mark theirs with the colour their genotype
     // forces (no warp primitive inside: the groups' loci have lists of their
     // own lengths)
+#pragma unroll 1
     for (int x = gl; x < nfa; x += G) {
         Lb[x] = x << 1;
         fl[x] = 0;
@@ -1978,6 +1985,7 @@ __device__ __forceinline__ float fagw_like(const ProblemDev& P, const FagwTables
     cp_async_wait_all();   // this lane's copies of the list; the barrier makes the group's visible
     __syncwarp();
     int clash = 0;
+#pragma unroll 1
     for (int x = nhet + gl; x < ntyp; x += G) {
         const int ent = typ[x], i = ent >> 2, g = ent & 3;
         const int bits = g == G_HOMOZ_A ? 3 : 5;   // used, fixed A / fixed B
@@ -2003,8 +2011,10 @@ __device__ __forceinline__ float fagw_like(const ProblemDev& P, const FagwTables
     // end fixes the other to the opposite colour, in rounds until nothing
     // changes (at most kFagRounds): most edges then have both ends fixed, and
     // a fixed allele's colour is its component's, so its term is the same.
+#pragma unroll 1
     for (int round = 0; round < kFagRounds; ++round) {
         int changed = 0;
+#pragma unroll 1
         for (int q = gl; q < nhet; q += G) {
             const int i = typ[q] >> 2;
             const int u = e[2 * i], v = e[2 * i + 1];
@@ -2019,6 +2029,7 @@ __device__ __forceinline__ float fagw_like(const ProblemDev& P, const FagwTables
         if (!__any_sync(FULLMASK, changed)) break;   // the whole warp, as its groups share the loop
     }
     int bad = clash;
+#pragma unroll 1
     for (int q = gl; q < nhet; q += G) {
         const int i = typ[q] >> 2;   // the heterozygotes lead the list
         const int u = e[2 * i], v = e[2 * i + 1];
@@ -2061,6 +2072,7 @@ __device__ __forceinline__ float fagw_like(const ProblemDev& P, const FagwTables
     int zero = 0, forest = 0;
     const float lmaj = lfreq.x, lmin = lfreq.y;
     if (!bad)
+#pragma unroll 1
         for (int x = gl; x < nfa; x += G) {
             const int f = fl[x];
             if (!(f & 1)) continue;
@@ -2083,6 +2095,7 @@ __device__ __forceinline__ float fagw_like(const ProblemDev& P, const FagwTables
     forest = grp.any(forest);   // no union: every term is in already
     __syncwarp();
     if (!bad && forest) {
+#pragma unroll 1
         for (int x = gl; x < nfa; x += G) {
             const int c = cnt[x];
             const int n = (c >> 16) & 0x1fff, even = c & 0xffff;
@@ -2320,17 +2333,19 @@ __device__ __forceinline__ void filter_locus(float q0, float q1, float t, float 
 }
 
 // a locus's decision map from its filtered pair (both non-zero) and its draw;
-// t: the recombination fraction to the locus above (last: none above)
-__device__ __forceinline__ int locus_map(float f0, float f1, double u, bool last, float t) {
+// t: the recombination fraction to the locus above (last: none above).  U is
+// double, or float with the draw rounded down (Draws::get_rd): the same choices.
+template <typename U>
+__device__ __forceinline__ int locus_map(float f0, float f1, U u, bool last, float t) {
     if (last) {
-        const int v = (u < (double)(f0 / (f0 + f1))) ? 0 : 1;
+        const int v = (u < (U)(f0 / (f0 + f1))) ? 0 : 1;
         return v | (v << 1);
     }
     const float a = 1.f - t;
     const float x0 = f0 * a, y0 = f1 * t;   // next = 0
     const float x1 = f0 * t, y1 = f1 * a;   // next = 1
-    const int d0 = (u < (double)(x0 / (x0 + y0))) ? 0 : 1;
-    const int d1 = (u < (double)(x1 / (x1 + y1))) ? 0 : 1;
+    const int d0 = (u < (U)(x0 / (x0 + y0))) ? 0 : 1;
+    const int d1 = (u < (U)(x1 / (x1 + y1))) ? 0 : 1;
     return d0 | (d1 << 1);
 }
 
@@ -2653,6 +2668,33 @@ static bool msw_shape(const ProblemDev& P, int G, int eb, int cs, MswShape* out)
     return false;
 }
 
+// One of a meiosis's relatives (P.mrel) at 32 loci: its entry and the two bits
+// of its genotype codes.  Lane r of a warp holds relative r.
+struct Relative {
+    uint32_t entry, c0, c1;
+};
+__device__ __forceinline__ Relative load_relative(const ProblemDev& P, int m, int word, int lane) {
+    Relative r;
+    r.entry = P.mrel[(size_t)m * kRelatives + lane];
+    r.c0 = r.c1 = 0u;
+    if (r.entry != kNoRelative && word < P.mflip_words) {
+        const uint32_t* g = P.gplane + (size_t)(r.entry & 0xffffu) * 2 * P.mflip_words + word;
+        r.c0 = g[0];
+        r.c1 = g[P.mflip_words];
+    }
+    return r;
+}
+
+// relatives_rule at a warp's 32 loci: lane r holds relative r, lane l locus
+// l's column and the meiosis's own indicator tb there.
+__device__ __forceinline__ void flips_by_relatives(const ProblemDev& P, int m, const Relative& own,
+                                                   const uint32_t* col, int tb, uint32_t* same, uint32_t* never) {
+    relatives_rule(
+        m, P.F, __ballot_sync(FULLMASK, tb), [&](int r) { return __shfl_sync(FULLMASK, own.entry, r); },
+        [&](int r) { return __shfl_sync(FULLMASK, own.c0, r); }, [&](int r) { return __shfl_sync(FULLMASK, own.c1, r); },
+        [&](int b) { return __ballot_sync(FULLMASK, (col[b >> 5] >> (b & 31)) & 1u); }, same, never);
+}
+
 template <int G, typename E>
 __global__ void __launch_bounds__(kMswThreads, 1) msweep_kernel(ProblemDev P, MswShape sh, uint32_t* dg, int first,
                                                              const int32_t* order, int64_t ostride, int nm,
@@ -2685,12 +2727,15 @@ __global__ void __launch_bounds__(kMswThreads, 1) msweep_kernel(ProblemDev P, Ms
     const int32_t* ord = order + cr * ostride;
     const int nmw = sh.nl / 32, MW = P.mflip_words;
     if (sh.staged)
+#pragma unroll 1
         for (int i = tid; i < nl * W; i += NT) col[i] = gcol[i];
+#pragma unroll 1
     for (int i = tid; i <= nl; i += NT) th[i] = lo + i > 0 && lo + i < M ? P.c_theta_f[(size_t)chain * (M - 1) + lo + i - 1] : 0.f;
     auto load_masks = [&](int step) {   // both masks of the step's meiosis into its buffer
         if (step >= nm) return;
         const uint32_t* src = P.mflip + (size_t)ord[step] * 2 * MW;
         uint32_t* dst = msk + (step & 1) * 2 * nmw;
+#pragma unroll 1
         for (int i = tid; i < 2 * nmw; i += NT) {
             const int k = i >= nmw, w = (k ? i - nmw : i) + (lo >> 5);
             dst[i] = w < MW ? src[k * MW + w] : 0u;
@@ -2700,6 +2745,7 @@ __global__ void __launch_bounds__(kMswThreads, 1) msweep_kernel(ProblemDev P, Ms
     if (tid < 3) ctl[tid] = 0;
     __syncthreads();
     // the likelihood of every column as it is
+#pragma unroll 1
     for (int h = warp * kLoci; h < nl; h += (NT >> 5) * kLoci) {
         const int i = h + lane / G;
         const bool valid = i < nl;
@@ -2717,20 +2763,29 @@ __global__ void __launch_bounds__(kMswThreads, 1) msweep_kernel(ProblemDev P, Ms
     const int vw = rank * sh.vpb + warp;                  // this warp's virtual warp
     const bool scans = warp < sh.vpb && vw < nw;
     const int s0 = min(M, (vw * 32 + lane) * L) - lo, s1 = min(M, (vw * 32 + lane + 1) * L) - lo;   // its run of loci
+    // the genotypes of a step's relatives at this warp's first 32 loci, read a step ahead
+    Relative next = load_relative(P, nm > 0 ? ord[0] : 0, (lo + warp * 32) >> 5, lane);
+#pragma unroll 1
     for (int j = 0; j < nm; ++j) {
         const int m = ord[j], mw = m >> 5, mb = m & 31;
         // the step's pairs: from the genotypes where they decide, else listed
         const uint32_t* em = msk + (j & 1) * 2 * nmw;
+#pragma unroll 1
         for (int i0 = warp * 32; i0 < nl; i0 += NT) {
             const int i = i0 + lane;
-            bool hard = false;
-            if (i < nl) {
-                const float keep = cur[i];
-                const int tb = (col[(size_t)i * W + mw] >> mb) & 1;
-                const bool same = (em[i0 >> 5] >> lane) & 1, never = (em[nmw + (i0 >> 5)] >> lane) & 1;
-                hard = keep == -INFINITY || !(same || never);
-                tog[i] = same ? keep : -INFINITY;
-                pr[i] = same ? make_float2(1.f, 1.f) : make_float2(tb ? 0.f : 1.f, tb ? 1.f : 0.f);
+            const bool in = i < nl;
+            const float keep = in ? cur[i] : 0.f;
+            const uint32_t* mine = col + (size_t)(in ? i : i0) * W;
+            const int tb = (mine[mw] >> mb) & 1;
+            uint32_t same = em[i0 >> 5], never = em[nmw + (i0 >> 5)];
+            if (__any_sync(FULLMASK, in && !(((same | never) >> lane) & 1)))
+                flips_by_relatives(P, m, i0 == warp * 32 ? next : load_relative(P, m, (lo + i0) >> 5, lane), mine,
+                                   tb, &same, &never);
+            const bool sm = (same >> lane) & 1, nv = (never >> lane) & 1;
+            const bool hard = in && (keep == -INFINITY || !(sm || nv));
+            if (in) {
+                tog[i] = sm ? keep : -INFINITY;
+                pr[i] = sm ? make_float2(1.f, 1.f) : make_float2(tb ? 0.f : 1.f, tb ? 1.f : 0.f);
             }
             const unsigned b = __ballot_sync(FULLMASK, hard);
             int at = 0;
@@ -2739,9 +2794,11 @@ __global__ void __launch_bounds__(kMswThreads, 1) msweep_kernel(ProblemDev P, Ms
             if (hard) list[at + __popc(b & ((1u << lane) - 1u))] = (uint16_t)i;
         }
         load_masks(j + 1);
+        next = load_relative(P, j + 1 < nm ? ord[j + 1] : m, (lo + warp * 32) >> 5, lane);
         __syncthreads();
         const int nh = ctl[j & 1];
         if (tid == 0) ctl[(j + 1) & 1] = 0;
+#pragma unroll 1
         for (int h = warp * kLoci; h < nh; h += (NT >> 5) * kLoci) {
             const int k = h + lane / G;
             const bool valid = k < nh;
@@ -2764,6 +2821,7 @@ __global__ void __launch_bounds__(kMswThreads, 1) msweep_kernel(ProblemDev P, Ms
         // forward filter: run products, scanned within the warp, the warp totals passed to every block
         float p00 = 1.f, p01 = 0.f, p10 = 0.f, p11 = 1.f;
         if (scans) {
+#pragma unroll 1
             for (int i = s0; i < s1; ++i) {
                 const float2 q = pr[i];
                 filter_product(q.x, q.y, th[i], p00, p01, p10, p11);
@@ -2816,6 +2874,7 @@ __global__ void __launch_bounds__(kMswThreads, 1) msweep_kernel(ProblemDev P, Ms
                 v0 = vw > 0 ? __fadd_rn(below.x, below.y) : 1.f;
                 v1 = vw > 0 ? __fadd_rn(below.z, below.w) : 1.f;
             }
+#pragma unroll 1
             for (int i = s0; i < s1; ++i) {
                 const float2 q = pr[i];
                 float f0, f1;
@@ -2849,7 +2908,9 @@ __global__ void __launch_bounds__(kMswThreads, 1) msweep_kernel(ProblemDev P, Ms
         if (bad) break;   // every block of the cluster leaves here together
         if (scans) {
             int rel = x - cnt;   // draws above this run in the block
+#pragma unroll 1
             for (int v = vw + 1; v < min(nw, (rank + 1) * sh.vpb); ++v) rel += wcnt[v] & 0x3fffffff;
+#pragma unroll 1
             for (int i = s1 - 1; i >= s0; --i) {
                 const float2 f = pr[i];
                 didx[i] = rel;
@@ -2857,17 +2918,19 @@ __global__ void __launch_bounds__(kMswThreads, 1) msweep_kernel(ProblemDev P, Ms
             }
         }
         __syncthreads();
+#pragma unroll 1
         for (int i = tid; i < nl; i += NT) {
             const float2 f = pr[i];
             int dmap;
             if (f.x == 0.f) dmap = 3;
             else if (f.y == 0.f) dmap = 0;
-            else dmap = locus_map(f.x, f.y, draws.get(cr, chain, j, above + didx[i]), lo + i == M - 1, th[i + 1]);
+            else dmap = locus_map(f.x, f.y, draws.get_rd(cr, chain, j, above + didx[i]), lo + i == M - 1, th[i + 1]);
             maps[i] = (uint8_t)dmap;
         }
         __syncthreads();
         int xm = 2;   // identity: bit0 = 0, bit1 = 1
         if (scans) {
+#pragma unroll 1
             for (int i = s1 - 1; i >= s0; --i) xm = map_compose(maps[i], xm);
             // suffix composition within the warp
             for (int d = 1; d < 32; d <<= 1) {
@@ -2890,6 +2953,7 @@ __global__ void __launch_bounds__(kMswThreads, 1) msweep_kernel(ProblemDev P, Ms
             int in = __shfl_down_sync(FULLMASK, map_compose(xm, tail), 1);
             if (lane == 31) in = tail;
             int sv = in & 1;
+#pragma unroll 1
             for (int i = s1 - 1; i >= s0; --i) {
                 sv = (maps[i] >> sv) & 1;
                 const uint32_t w = col[(size_t)i * W + mw];
@@ -2903,6 +2967,7 @@ __global__ void __launch_bounds__(kMswThreads, 1) msweep_kernel(ProblemDev P, Ms
     }
     __syncthreads();
     if (sh.staged)
+#pragma unroll 1
         for (int i = tid; i < nl * W; i += NT) gcol[i] = col[i];
 }
 

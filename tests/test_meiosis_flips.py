@@ -36,11 +36,12 @@ def family(members, loops, markers, untyped, missing, seed):
     return g
 
 
-def flips(g):
+def flips(g, dg=None):
     prob = api.Problem.from_arrays(g, with_legal=False)
     desc = prob.desc()
     out = np.zeros((2 * (g["N"] - g["F"]), g["M"]), np.uint8)
-    assert api.lib().sl_problem_meiosis_flips(ctypes.byref(desc), out.ctypes.data_as(ctypes.c_void_p)) == 0
+    at = None if dg is None else dg.ctypes.data_as(ctypes.c_void_p)
+    assert api.lib().sl_problem_meiosis_flips(ctypes.byref(desc), at, out.ctypes.data_as(ctypes.c_void_p)) == 0
     return out
 
 
@@ -81,6 +82,40 @@ def test_flips_follow_from_the_genotypes(members, loops, markers, untyped, missi
                 else:
                     dg[l, person, par] ^= 1
     assert decided > 0
+
+
+@pytest.mark.parametrize("members,loops,markers,untyped,missing,seed", [
+    (12, 0, 33, 0.0, 0.0, 1), (30, 1, 64, 0.0, 0.3, 2), (40, 3, 31, 0.3, 0.1, 3), (60, 2, 32, 0.6, 0.05, 4),
+    (110, 4, 40, 0.1, 0.5, 5), (110, 3, 65, 0.0, 0.05, 6)])
+def test_flips_that_follow_from_the_graph(members, loops, markers, untyped, missing, seed):
+    """The same with the graph's own meioses (relatives' alleles), on the gene
+    drop's graph and on three graphs moved away from it by legal toggles."""
+    g = family(members, loops, markers, untyped, missing, seed)
+    P = port.Port(dict(g, legal=np.full((g["M"], g["N"]), 15, np.uint8), trait_prior=np.zeros((g["M"], g["N"], 4))))
+    rng = np.random.default_rng(seed + 200)
+    dg = np.ascontiguousarray(g["dg0"], np.int32)
+    alone = flips(g)
+    for graph in range(4):
+        rule = flips(g, dg)
+        assert not np.any(rule == 3) and np.array_equal(rule[alone != 0], alone[alone != 0])
+        assert members < 30 or ((rule != 0) & (alone == 0)).any()
+        for m, l in zip(*np.nonzero((rule != 0) & (alone == 0))):
+            person, par = g["F"] + m // 2, m % 2
+            base = P.fag(dg, int(l))
+            dg[l, person, par] ^= 1
+            lk = P.fag(dg, int(l))
+            dg[l, person, par] ^= 1
+            assert base > 0.0
+            if rule[m, l] == 1:
+                assert abs(lk - base) <= 1e-12 * base, (m, l)
+            else:
+                assert lk == 0.0, (m, l)
+        for l in range(g["M"]):   # another legal graph
+            for m in rng.permutation(rule.shape[0]):
+                person, par = g["F"] + m // 2, m % 2
+                dg[l, person, par] ^= 1
+                if rng.random() < 0.5 or P.fag(dg, l) == 0.0:
+                    dg[l, person, par] ^= 1
 
 
 @pytest.mark.gpu
