@@ -70,7 +70,8 @@ std::string jit_source(const JitProgramIn& in, int threads, bool shared) {
     s.reserve(in.n_words * 24 + 4096);
     const int64_t npos = (int64_t)(in.M - 1) * in.n;
     emitf(s, "#define S %d\n", threads);
-    s += "typedef unsigned int u32;\n";
+    s += "typedef unsigned int u32;\n"
+         "#ifdef __CUDA_ARCH__\n#define TOGETHER() __syncthreads()\n#else\n#define TOGETHER()\n#endif\n";
     emitf(s,
           "extern \"C\" __global__ void __launch_bounds__(S) sl_lod_jit(const u32* __restrict__ graphs, long long gw,\n"
           "    int G, double* __restrict__ vals, int* status, const float* __restrict__ partial,\n"
@@ -78,7 +79,10 @@ std::string jit_source(const JitProgramIn& in, int threads, bool shared) {
     if (shared) s += "  extern __shared__ float sh[];\n  float* A = sh + threadIdx.x;\n";
     emitf(s, "  const long long npos = %lldLL;\n", (long long)npos);
     s += "  const long long ntask = (long long)G * npos;\n";
-    s += "  for (long long t = (long long)blockIdx.x * S + threadIdx.x; t < ntask; t += (long long)gridDim.x * S) {\n";
+    // the whole block goes through the loop together: threads past the last task repeat it and write nothing
+    s += "  for (long long t0 = (long long)blockIdx.x * S; t0 < ntask; t0 += (long long)gridDim.x * S) {\n"
+         "    const bool mine = t0 + threadIdx.x < ntask;\n"
+         "    const long long t = mine ? t0 + threadIdx.x : ntask - 1;\n";
     emitf(s, "    const int b = (int)(t / npos);\n    const int pidx = (int)(t %% npos);\n");
     emitf(s, "    const int l = pidx / %d, o = pidx %% %d;\n", in.n, in.n);
     emitf(s, "    const u32* cL = graphs + (long long)b * gw + (long long)l * %d;\n    const u32* cR = cL + %d;\n", in.W,
@@ -193,6 +197,7 @@ std::string jit_source(const JitProgramIn& in, int threads, bool shared) {
             for (int q = 0; q < cnt; ++q)
                 emitf(s, "      %s = ldexpf(%s, -e%d);\n", news[q].c_str(), olds[q].c_str(), k);
             s += "    }\n";
+            if (k % 4 == 3) s += "    TOGETHER();\n";
         } else {   // LI_END
             const int rs = pc[1];
             result = rs >= 0 ? ref(rs) : std::string("0.0f");
@@ -209,7 +214,7 @@ std::string jit_source(const JitProgramIn& in, int threads, bool shared) {
           "    else v = (double)logf(result) + (double)scale * 0.69314718055994530942 - rec - (%.17g);\n",
           in.zero_ok ? "" : ("atomicCAS(status, 0, " + std::to_string((int)ST_LOD_NONPOS) + ");").c_str(),
           in.marker_trans);
-    s += "    vals[t] = v;\n  }\n}\n";
+    s += "    if (mine) vals[t] = v;\n  }\n}\n";
     return s;
 }
 

@@ -21,6 +21,14 @@ struct JitProgramIn {
     int zero_ok;             // a zero trait likelihood is a zero term, not an error
 };
 
+// Threads per block of the scorer with its values in registers.  A block's
+// warps start together and so fetch the straight-line code together: 64 graphs
+// of the 120-member pedigree (146 slots) took 0.60 ms in blocks of 128, 0.32
+// in blocks of 512 (4 graphs 67 and 36 us).  With many slots the 128 registers
+// a thread that such a block leaves are too few: 731 slots (400 members) 0.71
+// ms in blocks of 128, 0.93 in blocks of 512.
+inline int jit_lod_threads(int slots) { return slots <= 192 ? 512 : 128; }
+
 struct JitLod {
     void* lib = nullptr;     // cudaLibrary_t
     void* kern = nullptr;    // cudaKernel_t
