@@ -188,6 +188,7 @@ struct sl_ctx {
     std::vector<int32_t> adj_prevs;
     size_t adj_budget = 0;            // shared bytes per warp the plan must fit (0: the default)
     double* d_adjG = nullptr;        // [chunk][6] gradients
+    double* d_ptrait = nullptr;      // [6] log P(T)'s
     int64_t adj_chunk = 0;
     // the adjoint's forms: one warp per task with its matrices in shared memory, one thread per
     // task with them in a global arena (a column per thread), or the peel's adjoint compiled for
@@ -2937,6 +2938,7 @@ static int adjoint_choose(sl_ctx* ctx, const uint32_t* graphs, int64_t words, in
         for (const AdjJit& j : ctx->adj_jit_v)
             if ((rc = adjoint_jit_arena(ctx, nt, j))) return rc;
     int st = 0;
+    CK(cudaStreamSynchronize(ctx->lstream));   // log P(T)'s gradient may still report there
     CK(cudaStreamSynchronize(ctx->stream));
     CK(cudaMemcpy(&st, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost));
     cudaEvent_t a = take_event(ctx), b = take_event(ctx);
@@ -2981,16 +2983,26 @@ int sl_trait_backward(sl_ctx* ctx, int32_t n_graphs, const int32_t* dgs, double*
     const int64_t npos = (int64_t)(P.M - 1) * P.n_lod;
     CK(cudaSetDevice(ctx->device));
     int rc;
+    // log P(T)'s gradient, one warp's work (0.4 ms on the 120-member pedigree),
+    // beside the graphs' on the second stream, into a buffer of its own
     if (ptrait_grad) {
-        if ((rc = adjoint_chunk(ctx, 1))) return rc;
-        Prof pr(ctx, SL_KERNEL_LOD);
-        CK(launch_trait_adjoint(P, ctx->adj, nullptr, 0, 0, 1, ctx->d_adjG, ctx->d_status, ctx->stream, ctx->sms));
-        double g6[6];
-        CK(cudaMemcpyAsync(g6, ctx->d_adjG, sizeof(g6), cudaMemcpyDeviceToHost, ctx->stream));
-        if ((rc = sl_synchronize(ctx))) return rc;
-        for (int k = 0; k < 4; ++k) ptrait_grad[k] = g6[2 + k];
+        if (!ctx->d_ptrait && (rc = dev_alloc(ctx, &ctx->d_ptrait, 6))) return rc;
+        CK(cudaEventRecord(ctx->ev_fork, ctx->stream));   // after what is queued there: the status word is one
+        CK(cudaStreamWaitEvent(ctx->lstream, ctx->ev_fork, 0));
+        Prof pr(ctx, SL_KERNEL_LOD, ctx->lstream);
+        CK(launch_trait_adjoint(P, ctx->adj, nullptr, 0, 0, 1, ctx->d_ptrait, ctx->d_status, ctx->lstream, ctx->sms));
     }
-    if (n_graphs == 0) return SL_OK;
+    auto ptrait = [&]() -> int {   // read once both streams are done
+        if (!ptrait_grad) return SL_OK;
+        double g6[6];
+        CK(cudaMemcpy(g6, ctx->d_ptrait, sizeof(g6), cudaMemcpyDeviceToHost));
+        for (int k = 0; k < 4; ++k) ptrait_grad[k] = g6[2 + k];
+        return SL_OK;
+    };
+    if (n_graphs == 0) {
+        if ((rc = sl_synchronize(ctx))) return rc;
+        return ptrait();
+    }
     if (n_graphs > ctx->graphs_cap) {
         if (ctx->d_graphs) {
             cudaStreamSynchronize(ctx->stream);
@@ -3020,7 +3032,8 @@ int sl_trait_backward(sl_ctx* ctx, int32_t n_graphs, const int32_t* dgs, double*
         CK(cudaMemcpyAsync(grad + t0 * 6, ctx->d_adjG, sizeof(double) * 6 * nt, cudaMemcpyDeviceToHost,
                            ctx->stream));
     }
-    return sl_synchronize(ctx);
+    if ((rc = sl_synchronize(ctx))) return rc;
+    return ptrait();
 }
 
 int sl_adjoint_memory(sl_ctx* ctx, int64_t bytes_per_task, int32_t* segments, int64_t* used_bytes) {
