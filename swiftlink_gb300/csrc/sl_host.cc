@@ -254,9 +254,9 @@ cudaEvent_t take_event(sl_ctx* c) {
 // Bracket one launch with events when profiling is on.
 // Kernels one M-sweep of nm meioses launches for a chain: in the fast mode one
 // (a cluster per chain), else a reset, then per meiosis a likelihood and a
-// filter kernel.
+// filter kernel; in the exact mode the filter and the sampling are two.
 static int64_t msweep_kernels(const sl_ctx* ctx, int nm) {
-    if (ctx->sampler_precision == SL_SAMPLER_EXACT) return 1 + 2 * (int64_t)nm;
+    if (ctx->sampler_precision == SL_SAMPLER_EXACT) return 1 + 3 * (int64_t)nm;
     return msweep_launches(ctx->P, ctx->n_chains, nm);
 }
 

@@ -19,8 +19,9 @@
 //  * msweep_kernel<G>     -- fast mode: a chain's whole M-sweep by one cluster.
 //  * fag_warp_kernel<G>   -- fast-mode likelihoods in lane groups of G (chains
 //                            whose share of loci does not fit a cluster).
-//  * ffbs_kernel<T>       -- forward filter / backward sample of one meiosis,
-//                            one warp per chain, in the reference's order.
+//  * ffbs_exact_runs_kernel, ffbs_exact_kernel -- exact mode: forward filter of
+//                            one meiosis in runs that start anew, backward
+//                            sampling as a composition of choices.
 //  * ffbs_scan_kernel     -- the same as block-wide scans (fast mode).
 //  * loglik_*_kernel      -- log P(G, graph) of (graph, map) chain pairs (MC3).
 // Scorer:
@@ -2169,66 +2170,52 @@ struct Flt<double> {
     static __device__ __forceinline__ double sub(double a, double b) { return DSUB(a, b); }
     static __device__ __forceinline__ double div(double a, double b) { return DDIV(a, b); }
 };
-template <>
-struct Flt<float> {
-    static __device__ __forceinline__ float mul(float a, float b) { return a * b; }
-    static __device__ __forceinline__ float add(float a, float b) { return a + b; }
-    static __device__ __forceinline__ float sub(float a, float b) { return a - b; }
-    static __device__ __forceinline__ float div(float a, float b) { return __fdividef(a, b); }
-};
 
-// One warp per chain.  All 32 lanes run the same serial recursion on values
-// broadcast by shuffles from coalesced 32-locus chunks (the FP64 pipe costs
-// the same per warp instruction whatever the active mask).  T=double is the
-// reference's arithmetic; T=float is the fast filter on normalised pairs.
-template <typename T>
-__global__ void __launch_bounds__(32) ffbs_kernel(ProblemDev P, uint32_t* dg, int first, int nchain,
-                                                  const int32_t* order, int64_t ostride, int step, Draws draws,
-                                                  const uint8_t* sel, int want, const uint8_t* badc,
-                                                  const double* raw64, const float* raw32, T* fbbuf) {
-    using Fl = Flt<T>;
-    const int cr = blockIdx.x;
-    if (cr >= nchain) return;
-    if (sel && sel[cr] != want) return;
-    if (badc[cr]) return;
-    const int lane = threadIdx.x;
-    const int chain = first + cr;
-    const int m = order[cr * ostride + step];
-    uint32_t* G = dg + (size_t)chain * P.M * P.W;
-    T* fb = fbbuf + (size_t)cr * 2 * P.M;
-    const double* r64 = raw64 + (size_t)cr * 2 * P.M;
-    const float* r32 = raw32 ? raw32 + (size_t)cr * 2 * P.M : nullptr;
-    // forward filter (meiosis_sampler.cc:136-155)
-    T prev0 = (T)0, prev1 = (T)0;
+// one locus of the exact filter (meiosis_sampler.cc:136-155): the pair (f0, f1)
+// entering it becomes its own; th the recombination fraction below it
+__device__ __forceinline__ void exact_filter(double a0, double a1, double th, bool bottom, double& f0, double& f1) {
+    using Fl = Flt<double>;
+    double g0 = a0, g1 = a1;
+    if (!bottom) {
+        const double ax = Fl::sub(1.0, th);
+        g0 = Fl::mul(a0, Fl::add(Fl::mul(f1, th), Fl::mul(f0, ax)));
+        g1 = Fl::mul(a1, Fl::add(Fl::mul(f0, th), Fl::mul(f1, ax)));
+    }
+    const double tot = Fl::add(g0, g1);
+    f0 = Fl::div(g0, tot);
+    f1 = Fl::div(g1, tot);
+}
+
+// (x o y)(v) = x(y(v)) for 2-bit maps
+__device__ __forceinline__ int map_compose(int x, int y) {
+    const int y0 = y & 1, y1 = (y >> 1) & 1;
+    return ((x >> y0) & 1) | (((x >> y1) & 1) << 1);
+}
+
+// The exact filter and sampling of one meiosis by one warp, in the reference's
+// order (meiosis_sampler.cc:136-203): all 32 lanes run the same serial recursion
+// on values broadcast by shuffles from coalesced 32-locus chunks (the FP64 pipe
+// costs the same per warp instruction whatever the active mask).  For the
+// chains that ffbs_exact_kernel cannot split.
+__device__ void ffbs_serial_chain(const ProblemDev& P, uint32_t* G, int chain, int cr, int m, int step, const Draws& draws,
+                                  const double* r64, double* fb) {
+    using Fl = Flt<double>;
+    const int lane = threadIdx.x & 31;
+    double prev0 = 0.0, prev1 = 0.0;
     for (int base = 0; base < P.M; base += 32) {
         const int i = base + lane;
-        T q0 = (T)0, q1 = (T)0, th = (T)0;
+        double q0 = 0.0, q1 = 0.0, th = 0.0;
         if (i < P.M) {
-            if (sizeof(T) == 8) { q0 = (T)r64[2 * i]; q1 = (T)r64[2 * i + 1]; }
-            else { q0 = (T)r32[2 * i]; q1 = (T)r32[2 * i + 1]; }
-            if (i >= 1) th = (T)P.c_theta[(size_t)chain * (P.M - 1) + i - 1];
+            q0 = r64[2 * i];
+            q1 = r64[2 * i + 1];
+            if (i >= 1) th = P.c_theta[(size_t)chain * (P.M - 1) + i - 1];
         }
         const int n = min(32, P.M - base);
-        T k0 = (T)0, k1 = (T)0;
+        double k0 = 0.0, k1 = 0.0;
         for (int x = 0; x < n; ++x) {
-            const T a0 = __shfl_sync(FULLMASK, q0, x), a1 = __shfl_sync(FULLMASK, q1, x);
-            const T tx = __shfl_sync(FULLMASK, th, x);
-            T f0, f1;
-            if (base + x == 0) {
-                const T tot = Fl::add(a0, a1);
-                f0 = Fl::div(a0, tot);
-                f1 = Fl::div(a1, tot);
-            } else {
-                const T ax = Fl::sub((T)1, tx);
-                f0 = Fl::mul(a0, Fl::add(Fl::mul(prev1, tx), Fl::mul(prev0, ax)));
-                f1 = Fl::mul(a1, Fl::add(Fl::mul(prev0, tx), Fl::mul(prev1, ax)));
-                const T tt = Fl::add(f0, f1);
-                f0 = Fl::div(f0, tt);
-                f1 = Fl::div(f1, tt);
-            }
-            prev0 = f0;
-            prev1 = f1;
-            if (lane == x) { k0 = f0; k1 = f1; }
+            const double a0 = __shfl_sync(FULLMASK, q0, x), a1 = __shfl_sync(FULLMASK, q1, x);
+            exact_filter(a0, a1, __shfl_sync(FULLMASK, th, x), base + x == 0, prev0, prev1);
+            if (lane == x) { k0 = prev0; k1 = prev1; }
         }
         if (i < P.M) { fb[2 * i] = k0; fb[2 * i + 1] = k1; }
     }
@@ -2241,8 +2228,8 @@ __global__ void __launch_bounds__(32) ffbs_kernel(ProblemDev P, uint32_t* dg, in
         const int n = top - lo + 1;
         const int i = top - lane;
         const bool in = i >= lo;
-        const T f0 = in ? fb[2 * i] : (T)0, f1 = in ? fb[2 * i + 1] : (T)0;
-        const T th = (in && i < P.M - 1) ? (T)P.c_theta[(size_t)chain * (P.M - 1) + i] : (T)0;
+        const double f0 = in ? fb[2 * i] : 0.0, f1 = in ? fb[2 * i + 1] : 0.0;
+        const double th = (in && i < P.M - 1) ? P.c_theta[(size_t)chain * (P.M - 1) + i] : 0.0;
         uint32_t* wp = in ? (G + (size_t)i * P.W + (m >> 5)) : nullptr;
         const int cur = in ? (int)((*wp >> (m & 31)) & 1u) : 0;
         const int64_t c0 = cursor;
@@ -2250,25 +2237,164 @@ __global__ void __launch_bounds__(32) ffbs_kernel(ProblemDev P, uint32_t* dg, in
         int mine = cur;
         for (int x = 0; x < n; ++x) {
             const int ii = top - x;
-            T a0 = __shfl_sync(FULLMASK, f0, x), a1 = __shfl_sync(FULLMASK, f1, x);
-            const T tx = __shfl_sync(FULLMASK, th, x);
+            double a0 = __shfl_sync(FULLMASK, f0, x), a1 = __shfl_sync(FULLMASK, f1, x);
+            const double tx = __shfl_sync(FULLMASK, th, x);
             if (ii < P.M - 1) {
-                const T ax = Fl::sub((T)1, tx);
+                const double ax = Fl::sub(1.0, tx);
                 a0 = Fl::mul(a0, nxt != 0 ? tx : ax);
                 a1 = Fl::mul(a1, nxt != 1 ? tx : ax);
             }
             int samp;
-            if (a0 == (T)0) samp = 1;
-            else if (a1 == (T)0) samp = 0;
+            if (a0 == 0.0) samp = 1;
+            else if (a1 == 0.0) samp = 0;
             else {
                 const double r = __shfl_sync(FULLMASK, dr, (int)(cursor - c0));
                 ++cursor;
-                samp = (r < (double)Fl::div(a0, Fl::add(a0, a1))) ? 0 : 1;
+                samp = (r < Fl::div(a0, Fl::add(a0, a1))) ? 0 : 1;
             }
             nxt = samp;
             if (lane == x) mine = samp;
         }
         if (in && mine != cur) *wp ^= (1u << (m & 31));
+    }
+}
+
+// The exact filter, split where it starts anew.  A locus where one of the two
+// likelihoods is zero leaves the pair (0, 1) or (1, 0), exactly, whatever came
+// before: 0 x / (0 x + a y) is 0 and a y / (0 + a y) is 1 for finite x and any
+// a y > 0.  So a run of loci from one such locus to the next is filtered by
+// itself, the same operations on the same values, and the runs side by side: a
+// warp's lanes each take the run that starts at their locus.  That holds while
+// no product underflows; loci whose larger likelihood, or whose smaller
+// non-zero filtered value, lies below kExactTiny set the chain's flag, and
+// ffbs_exact_kernel then does it all in one run.  The serial recursion is
+// bound by the latency of FP64 (about 900 cycles a locus, two divisions and
+// five dependent operations): an M-sweep of two chains of 30 members took 13.7
+// ms at 200 SNPs and 121 ms at 2,000, in runs 2.6 and 3.6 ms; one of 120
+// members and 2,000 SNPs 549 and 36 ms.
+constexpr double kExactTiny = 1e-280;
+
+__global__ void __launch_bounds__(32) ffbs_exact_runs_kernel(ProblemDev P, int first, int nchain, const uint8_t* sel,
+                                                             int want, const uint8_t* badc, const double* raw64,
+                                                             double* fbbuf, int* flag, int64_t fstride) {
+    const int cr = blockIdx.y, M = P.M;
+    if (sel && sel[cr] != want) return;
+    if (badc[cr]) return;
+    const int chain = first + cr, i = blockIdx.x * 32 + threadIdx.x;
+    if (i >= M) return;
+    const double* r = raw64 + (size_t)cr * 2 * M;
+    double* fb = fbbuf + (size_t)cr * 2 * M;
+    const double* th = P.c_theta + (size_t)chain * (M - 1);
+    auto anew = [&](double a0, double a1) { return (a0 == 0.0) != (a1 == 0.0); };
+    double a0 = r[2 * i], a1 = r[2 * i + 1];
+    if (i > 0 && !anew(a0, a1)) return;   // in another lane's run
+    double f0 = 0.0, f1 = 0.0;
+    bool tiny = false;
+    for (int k = i;; ) {
+        tiny |= !(fmax(a0, a1) >= kExactTiny);
+        if (k > 0 && k == i) {
+            f0 = a0 == 0.0 ? 0.0 : 1.0;
+            f1 = a0 == 0.0 ? 1.0 : 0.0;
+            tiny |= !(th[k - 1] >= 1e-20);
+        } else {
+            exact_filter(a0, a1, k > 0 ? th[k - 1] : 0.0, k == 0, f0, f1);
+        }
+        tiny |= (f0 != 0.0 && !(f0 >= kExactTiny)) || (f1 != 0.0 && !(f1 >= kExactTiny));
+        fb[2 * k] = f0;
+        fb[2 * k + 1] = f1;
+        if (++k >= M) break;
+        a0 = r[2 * k];
+        a1 = r[2 * k + 1];
+        if (anew(a0, a1)) break;
+    }
+    if (tiny) atomicOr(flag + cr * fstride, 1);
+}
+
+// Backward sampling of one meiosis over the filtered pairs, one block per
+// chain: a locus's choice given the one above, for both of that one's values,
+// is worked out at all loci at once (a locus draws when both its filtered
+// values are non-zero, so a suffix count gives each its draw), and the choices
+// are composed from the top.  The chain's flag (see above) sends it through
+// ffbs_serial_chain instead, and is cleared for the next meiosis.
+__global__ void __launch_bounds__(512) ffbs_exact_kernel(ProblemDev P, uint32_t* dg, int first, int nchain,
+                                                         const int32_t* order, int64_t ostride, int step, Draws draws,
+                                                         const uint8_t* sel, int want, const uint8_t* badc,
+                                                         const double* raw64, double* fbbuf, uint8_t* mapbuf, int* flag,
+                                                         int64_t fstride) {
+    __shared__ int wcnt[16], wmap[17];
+    using Fl = Flt<double>;
+    const int cr = blockIdx.x, M = P.M;
+    if (sel && sel[cr] != want) return;
+    if (badc[cr]) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+    const int chain = first + cr, m = order[cr * ostride + step];
+    uint32_t* G = dg + (size_t)chain * M * P.W;
+    double* fb = fbbuf + (size_t)cr * 2 * M;
+    uint8_t* maps = mapbuf + (size_t)cr * M;
+    const double* th = P.c_theta + (size_t)chain * (M - 1);
+    if (flag[cr * fstride]) {
+        if (warp == 0) ffbs_serial_chain(P, G, chain, cr, m, step, draws, raw64 + (size_t)cr * 2 * M, fb);
+        __syncthreads();
+        if (tid == 0) flag[cr * fstride] = 0;
+        return;
+    }
+    const int L = (M + blockDim.x - 1) / blockDim.x, s0 = min(M, tid * L), s1 = min(M, s0 + L);
+    int cnt = 0;
+    for (int i = s0; i < s1; ++i) cnt += fb[2 * i] != 0.0 && fb[2 * i + 1] != 0.0;
+    int x = cnt;   // draws of this run and those above it in the warp
+    for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_down_sync(FULLMASK, x, d);
+        if (lane + d < 32) x += y;
+    }
+    if (lane == 0) wcnt[warp] = x;
+    __syncthreads();
+    int idx = x - cnt;
+    for (int w = warp + 1; w < nw; ++w) idx += wcnt[w];
+    int g = 2;   // identity: bit 0 = 0, bit 1 = 1
+    for (int i = s1 - 1; i >= s0; --i) {
+        const double f0 = fb[2 * i], f1 = fb[2 * i + 1];
+        int map;
+        if (f0 == 0.0) map = 3;
+        else if (f1 == 0.0) map = 0;
+        else {
+            const double u = draws.get(cr, chain, step, idx++);
+            if (i == M - 1) {
+                map = (u < Fl::div(f0, Fl::add(f0, f1))) ? 0 : 3;
+            } else {
+                const double t = th[i], a = Fl::sub(1.0, t);
+                const double x0 = Fl::mul(f0, a), y0 = Fl::mul(f1, t);   // next = 0
+                const double x1 = Fl::mul(f0, t), y1 = Fl::mul(f1, a);   // next = 1
+                map = (u < Fl::div(x0, Fl::add(x0, y0)) ? 0 : 1) | (u < Fl::div(x1, Fl::add(x1, y1)) ? 0 : 2);
+            }
+        }
+        maps[i] = (uint8_t)map;
+        g = map_compose(map, g);
+    }
+    // suffix composition: within the warp, then across warps
+    for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_down_sync(FULLMASK, g, d);
+        if (lane + d < 32) g = map_compose(g, y);
+    }
+    if (lane == 0) wmap[warp] = g;
+    __syncthreads();
+    if (tid == 0) {
+        int acc = 2;
+        wmap[nw] = 2;
+        for (int w = nw - 1; w >= 0; --w) {
+            acc = map_compose(wmap[w], acc);
+            wmap[w] = acc;
+        }
+    }
+    __syncthreads();
+    const int tail = wmap[warp + 1];
+    int above = __shfl_down_sync(FULLMASK, map_compose(g, tail), 1);
+    if (lane == 31) above = tail;
+    int sv = above & 1;
+    for (int i = s1 - 1; i >= s0; --i) {
+        sv = (maps[i] >> sv) & 1;
+        uint32_t* wp = G + (size_t)i * P.W + (m >> 5);
+        const uint32_t w = *wp;
+        if (sv != (int)((w >> (m & 31)) & 1u)) *wp = w ^ (1u << (m & 31));
     }
 }
 
@@ -2287,12 +2413,6 @@ __device__ __forceinline__ void mat_norm(float& a, float& b, float& c, float& d)
         const float inv = 1.f / mx;
         a *= inv; b *= inv; c *= inv; d *= inv;
     }
-}
-
-// (x o y)(v) = x(y(v)) for 2-bit maps
-__device__ __forceinline__ int map_compose(int x, int y) {
-    const int y0 = y & 1, y1 = (y >> 1) & 1;
-    return ((x >> y0) & 1) | (((x >> y1) & 1) << 1);
 }
 
 // Block-wide scan scratch of ffbs_scan_kernel (blockDim.x = T, a multiple of 32, <= 1024).
@@ -4460,6 +4580,10 @@ static cudaError_t launch_msampler_t(const ProblemDev& P, uint32_t* dg, int firs
     }
     cudaError_t e0 = cudaMemsetAsync(badc, 0, (size_t)nchain, s);
     if (e0 != cudaSuccess) return e0;
+    if (exact) {   // the chains' flags (ffbs_exact_kernel), the first word of each one's part of ubuf
+        e0 = cudaMemset2DAsync(ubuf, sizeof(double) * P.M, 0, sizeof(int), (size_t)nchain, s);
+        if (e0 != cudaSuccess) return e0;
+    }
     const size_t smem = fag_block_bytes(P.N, P.F, fag_threads, fast);
     {
         cudaError_t e = ensure_smem((const void*)fag_kernel<IX, PP>, smem);
@@ -4504,10 +4628,14 @@ static cudaError_t launch_msampler_t(const ProblemDev& P, uint32_t* dg, int firs
             if (e != cudaSuccess) return e;
         }
         if (j < 0) continue;
-        if (exact)
-            ffbs_kernel<double><<<nchain, 32, 0, s>>>(P, dg, first, nchain, meioses, mstride, j, d, sel, want, badc,
-                                                      (const double*)raw, nullptr, (double*)fb);
-        else
+        if (exact) {
+            ffbs_exact_runs_kernel<<<dim3((unsigned)((P.M + 31) / 32), (unsigned)nchain), 32, 0, s>>>(
+                P, first, nchain, sel, want, badc, (const double*)raw, (double*)fb, (int*)ubuf, 2 * (int64_t)P.M);
+            const int bt = std::min(512, (P.M + 31) / 32 * 32);
+            ffbs_exact_kernel<<<nchain, bt, 0, s>>>(P, dg, first, nchain, meioses, mstride, j, d, sel, want, badc,
+                                                    (const double*)raw, (double*)fb, maps, (int*)ubuf,
+                                                    2 * (int64_t)P.M);
+        } else
             ffbs_scan_kernel<<<nchain, scan_threads, scan_smem, s>>>(P, dg, first, nchain, meioses, mstride, j, d, sel,
                                                                      want, badc, raw32, (float*)fb, maps, staged,
                                                                      upre);
