@@ -1114,6 +1114,28 @@ struct SlotAlloc {
     }
 };
 
+// Moves the ops' matrices (mat_off, and the offsets in the lists of previous
+// rfunctions) to where a matrix lies only from its op to the last op that reads
+// it; returns the cells that the peel then takes.
+int reuse_arena(std::vector<OpDev>& ops, std::vector<int32_t>& od) {
+    const int K = (int)ops.size();
+    std::vector<int> last(K);
+    for (int k = 0; k < K; ++k) {
+        last[k] = k;
+        for (int j = 0; j < ops[k].n_prev; ++j) last[od[ops[k].prev_ops_at + j]] = k;
+    }
+    last[K - 1] = K;   // the result
+    SlotAlloc sa;
+    for (int k = 0; k < K; ++k) {
+        ops[k].mat_off = sa.alloc(1 << (2 * ops[k].c));
+        for (int q = 0, at = ops[k].prev_at; q < ops[k].n_prev; ++q, at += 2 + od[at + 1])
+            od[at] = ops[od[ops[k].prev_ops_at + q]].mat_off;
+        for (int q = 0; q <= k; ++q)
+            if (last[q] == k) sa.release(ops[q].mat_off, 1 << (2 * ops[q].c));
+    }
+    return sa.high;
+}
+
 int phased_trait_host(int m, int p, int i, int j) {
     const int ma = (m == AA) || (m == AU && i == 0) || (m == UA && i == 1);
     const int pa = (p == AA) || (p == AU && j == 0) || (p == UA && j == 1);
@@ -1785,8 +1807,13 @@ int sl_create(const sl_problem_desc* d, const sl_options* opt, sl_ctx** out) {
     }
     if ((rc = upload(ctx, (double**)&P.dprob, d->disease_prob, (size_t)4 * N))) return bail(rc);
     if ((rc = upload(ctx, (uint8_t**)&P.dmask, dmask.data(), N))) return bail(rc);
-    if ((rc = upload(ctx, (OpDev**)&P.ops, ops.data(), K))) return bail(rc);
-    if ((rc = upload(ctx, (int32_t**)&P.opdata, od.data(), od.size()))) return bail(rc);
+    {
+        std::vector<OpDev> dops = ops;
+        std::vector<int32_t> dod = od;
+        P.arena = reuse_arena(dops, dod);
+        if ((rc = upload(ctx, (OpDev**)&P.ops, dops.data(), K))) return bail(rc);
+        if ((rc = upload(ctx, (int32_t**)&P.opdata, dod.data(), dod.size()))) return bail(rc);
+    }
     P.opdata_n = (int32_t)od.size();
     // small operation tables are copied to every L-sampler block; large ones
     // (hundreds of members) would take residency from the arenas
@@ -1811,10 +1838,11 @@ int sl_create(const sl_problem_desc* d, const sl_options* opt, sl_ctx** out) {
         P.ls_spill_cells = P.ls_arena - P.ls_cap;
     }
     const size_t lsw = lsampler_smem_per_warp(P);
-    const size_t lodw = (size_t)arena * (ctx->lod_precision == SL_LOD_FP32_RESCALED ? 4 : 8);
-    if (lst + lsw > kSmemBudget || lodw > kSmemBudget)
+    const size_t lodw = ((size_t)P.arena + 16) * (ctx->lod_precision == SL_LOD_FP32_RESCALED ? 4 : 8);
+    const size_t lod_all = (size_t)arena * (ctx->lod_precision == SL_LOD_FP32_RESCALED ? 4 : 8);
+    if (lst + lsw > kSmemBudget || lod_all > kSmemBudget)
         return bail(fail(nullptr, SL_EINVAL, "peel sequence needs %zu bytes per task, above the shared-memory budget",
-                         std::max(lsw, lodw)));
+                         std::max(lsw, lod_all)));
     ctx->ls_wpb = (int)std::max<size_t>(1, std::min<size_t>(4, (kSmemBudget - lst) / lsw));
     ctx->lod_wpb = (int)std::max<size_t>(1, std::min<size_t>(4, kSmemBudget / lodw));
     const size_t per_sm = prop.sharedMemPerMultiprocessor;

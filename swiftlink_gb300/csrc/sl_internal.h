@@ -37,7 +37,7 @@ constexpr uint32_t kRelOfP = 1u << 16, kRelOfO = 1u << 17, kRelOfI = 1u << 18;
 // Everything a kernel needs about one problem; passed by value.
 struct ProblemDev {
     int32_t N, F, M, K, n_lod, Nnf, W;   // W = 32-bit words per descent-graph column
-    int32_t arena;                       // sum over ops of 4^c
+    int32_t arena;                       // cells of the trait peel's matrices, reused as they die (reuse_arena)
     int32_t ls_arena;                    // the L-sampler's compact rfunctions: the largest, over loci, sum over
                                          // ops of their cells in legal states (sl_kernels.cu, ls_locus)
     int32_t ls_cap;                      // the part of them a task keeps in shared memory (<= ls_arena)

@@ -25,8 +25,8 @@
 //  * ffbs_scan_kernel     -- the same as block-wide scans (fast mode).
 //  * loglik_*_kernel      -- log P(G, graph) of (graph, map) chain pairs (MC3).
 // Scorer:
-//  * lod_kernel<T,R>      -- trait peel at every (graph, interval, position), one
-//                            warp per task; T=double is the plain FP64 form,
+//  * lod_kernel<T,R,L>    -- trait peel at every (graph, interval, position), L
+//                            lanes per task; T=double is the plain FP64 form,
 //                            R=true rescales every rfunction by a power of two
 //                            and carries the exponent.
 //  * lod_prog_kernel      -- the FP32 rescaled peel as a slot-program
@@ -3132,17 +3132,30 @@ __device__ __forceinline__ int person_bits(const ProblemDev& P, const uint32_t* 
     return dgbit(colL, b) | (dgbit(colL, b + 1) << 1) | (dgbit(colR, b) << 2) | (dgbit(colR, b + 1) << 3);
 }
 
-template <typename T, bool RESCALE>
+// L lanes a position, which share the cells of its rfunctions.  The FP64 pipe
+// bounds it (16 cycles for a warp's instruction, however many lanes it has), so:
+// several positions to a warp, since a two-member cutset has 16 cells and many
+// have 4; the recombination terms of a child from 16 products made once a
+// position (four multiplications for each of a cell's four terms before); the
+// recombination sum from the count of crossovers (one lane's 2 (N - F) additions
+// before); and matrices that lie where a dead one lay (reuse_arena), for 28
+// warps to an SM instead of 8.  Four graphs of 45 members and 401 SNPs (8,000
+// positions): 0.92 ms with a warp a position; 0.58 with 16 lanes, 0.36 with the
+// products, 0.25 with the smaller arena, the pipe at 74%.
+template <typename T, bool RESCALE, int L>
 __global__ void __launch_bounds__(128) lod_kernel(ProblemDev P, const uint32_t* graphs, int64_t graph_words,
                                                   int G, double* vals, int* status) {
     using Ar = Arith<T>;
     extern __shared__ __align__(16) unsigned char smem[];
-    const int wpb = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    T* A = (T*)(smem + (size_t)warp * P.arena * sizeof(T));
+    const int per = blockDim.x / L, at = threadIdx.x / L, lane = threadIdx.x & (L - 1);
+    T* A = (T*)(smem + (size_t)at * (P.arena + 16) * sizeof(T));
+    T* quarter_rec = A + P.arena;   // [bits ^ (5 i | 10 j)]: a quarter of trait_rec(bits, i, j)
     const int n = P.n_lod;
     const int64_t npos = (int64_t)(P.M - 1) * n;
     const int64_t ntask = (int64_t)G * npos;
-    for (int64_t t = (int64_t)blockIdx.x * wpb + warp; t < ntask; t += (int64_t)gridDim.x * wpb) {
+    // at - at % (32 / L): a warp's positions go round together, those past the end on the last one's data
+    for (int64_t t0 = (int64_t)blockIdx.x * per + at; t0 - at % (32 / L) < ntask; t0 += (int64_t)gridDim.x * per) {
+        const int64_t t = min(t0, ntask - 1);
         const int b = (int)(t / npos);
         const int64_t pidx = t % npos;
         const int l = (int)(pidx / n), o = (int)(pidx % n);
@@ -3152,7 +3165,9 @@ __global__ void __launch_bounds__(128) lod_kernel(ProblemDev P, const uint32_t* 
         const double thd = DMUL(P.partial[l], (double)(o + 1));
         const double th2d = DMUL(P.partial[l], (double)(n + 1 - (o + 1)));
         const T th = (T)thd, an = (T)DSUB(1.0, thd), th2 = (T)th2d, an2 = (T)DSUB(1.0, th2d);
-        const T quarter = (T)0.25;
+        for (int e = lane; e < 16; e += L)
+            quarter_rec[e] = Ar::mul((T)0.25, trait_rec<T>(e, 0, 0, th, an, th2, an2));
+        __syncwarp();
         int scale = 0;
         for (int k = 0; k < P.K; ++k) {
             const OpDev op = P.ops[k];
@@ -3161,7 +3176,7 @@ __global__ void __launch_bounds__(128) lod_kernel(ProblemDev P, const uint32_t* 
             const double* trait = P.dprob + 4 * op.peel;
             T* out = A + op.mat_off;
             T mx = (T)0;
-            for (int cell = lane; cell < ncell; cell += 32) {
+            for (int cell = lane; cell < ncell; cell += L) {
                 bool valid = true;
                 for (int q = 0; q < op.c; ++q) valid &= ((P.dmask[cut[q]] >> digit(cell, q)) & 1) != 0;
                 T total = (T)0;
@@ -3183,7 +3198,7 @@ __global__ void __launch_bounds__(128) lod_kernel(ProblemDev P, const uint32_t* 
                                     tmp = Ar::mul(tmp, A[pd[0] + idx]);
                                     pd += 2 + pd[1];
                                 }
-                                tmp = Ar::mul(tmp, Ar::mul(quarter, trait_rec<T>(bits, i, j, th, an, th2, an2)));
+                                tmp = Ar::mul(tmp, quarter_rec[bits ^ (5 * i | 10 * j)]);
                                 total = Ar::add(total, tmp);
                             }
                     } else if (op.type == PARENT) {
@@ -3210,7 +3225,7 @@ __global__ void __launch_bounds__(128) lod_kernel(ProblemDev P, const uint32_t* 
                                 for (int i = 0; i < 2; ++i)
                                     for (int j = 0; j < 2; ++j) {
                                         if (phased_trait(mt, pt, i, j) != kt) continue;
-                                        ct = Ar::add(ct, Ar::mul(quarter, trait_rec<T>(bits, i, j, th, an, th2, an2)));
+                                        ct = Ar::add(ct, quarter_rec[bits ^ (5 * i | 10 * j)]);
                                     }
                                 cp = Ar::mul(cp, ct);
                             }
@@ -3239,7 +3254,7 @@ __global__ void __launch_bounds__(128) lod_kernel(ProblemDev P, const uint32_t* 
             }
             __syncwarp();
             if (RESCALE) {
-                for (int s = 16; s > 0; s >>= 1) {
+                for (int s = L / 2; s > 0; s >>= 1) {
                     const T o2 = __shfl_xor_sync(FULLMASK, mx, s);
                     mx = o2 > mx ? o2 : mx;
                 }
@@ -3247,24 +3262,25 @@ __global__ void __launch_bounds__(128) lod_kernel(ProblemDev P, const uint32_t* 
                     if constexpr (sizeof(T) == 8) {
                         const int e = ilogb(mx);
                         const T f = scalbn(1.0, -e);
-                        for (int cell = lane; cell < ncell; cell += 32) out[cell] *= f;
+                        for (int cell = lane; cell < ncell; cell += L) out[cell] *= f;
                         scale += e;
                     } else {
                         // FP32: the largest cell to 2^scale_to (LI_SCALE, sl_internal.h)
                         const int e = ilogbf(mx) - op.scale_to;
-                        for (int cell = lane; cell < ncell; cell += 32) out[cell] = ldexpf(out[cell], -e);
+                        for (int cell = lane; cell < ncell; cell += L) out[cell] = ldexpf(out[cell], -e);
                         scale += e;
                     }
                 }
                 __syncwarp();
             }
         }
-        if (lane == 0) {
-            const double r = (double)A[P.ops[P.K - 1].mat_off];
-            // DescentGraph::get_recombination_prob (descent_graph.cc:212-242)
-            const double lt = log(P.theta[l]), la = log(DSUB(1.0, P.theta[l]));
-            double rec = 0.0;
-            for (int bb = 0; bb < 2 * P.Nnf; ++bb) rec = DADD(rec, dgbit(colL, bb) != dgbit(colR, bb) ? lt : la);
+        // DescentGraph::get_recombination_prob (descent_graph.cc:212-242) by the count of crossovers
+        const double r = (double)A[P.ops[P.K - 1].mat_off];
+        int cross = 0;
+        for (int w = lane; w < P.W; w += L) cross += __popc(colL[w] ^ colR[w]);
+        for (int s = L / 2; s > 0; s >>= 1) cross += __shfl_xor_sync(FULLMASK, cross, s);
+        if (lane == 0 && t0 < ntask) {
+            const double rec = DADD(DMUL((double)cross, P.log_theta[l]), DMUL((double)(2 * P.Nnf - cross), P.log_itheta[l]));
             double v;
             if (r <= 0.0) {
                 if (!P.lod_zero_ok) set_status(status, ST_LOD_NONPOS);
@@ -4729,27 +4745,42 @@ cudaError_t launch_msampler(const ProblemDev& P, uint32_t* dg, int first, int nc
 
 size_t fag_smem(int N, int F, int threads, int fast) { return fag_block_bytes(N, F, threads, fast); }
 
+template <bool RESCALE, int L>
+static cudaError_t launch_lod_lanes(const ProblemDev& P, const uint32_t* graphs, int64_t graph_words, int G,
+                                    double* vals, int* status, cudaStream_t s, int grid_cap, int wpb) {
+    const int64_t ntask = (int64_t)G * (P.M - 1) * P.n_lod;
+    const size_t warp = (size_t)(32 / L) * (P.arena + 16) * sizeof(double);
+    wpb = (int)std::max<size_t>(1, std::min<size_t>(wpb, 100 * 1024 / warp));
+    const int per = wpb * (32 / L);
+    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(grid_cap, (ntask + per - 1) / per));
+    const void* k = (const void*)lod_kernel<double, RESCALE, L>;
+    const cudaError_t e = ensure_smem(k, wpb * warp);
+    if (e != cudaSuccess) return e;
+    lod_kernel<double, RESCALE, L><<<(int)grid, wpb * 32, wpb * warp, s>>>(P, graphs, graph_words, G, vals, status);
+    return cudaGetLastError();
+}
+
+// 16 lanes to a position, and 8 from 20,000 positions (128 to an SM, more than
+// the warps of 4 that are resident there): at 8 the FP64 pipe gives its whole
+// rate to fewer idle lanes, but a position takes half as long again.  16 | 8
+// lanes, plain form, 45 members: 1,000 positions 0.114 | 0.181 ms, 8,000 0.254 |
+// 0.274, 40,000 1.17 | 1.06; rescaled, 120 members: 5,000 0.94 | 1.00, 40,000
+// 6.4 | 5.7.  32 and 4 lanes are slower at every one of these but 40,000 of the
+// 45-member pedigree, where 4 measured as 8.
+template <bool RESCALE>
+static cudaError_t launch_lod64(const ProblemDev& P, const uint32_t* graphs, int64_t graph_words, int G, double* vals,
+                                int* status, cudaStream_t s, int grid_cap, int wpb) {
+    if ((int64_t)G * (P.M - 1) * P.n_lod >= 20000)
+        return launch_lod_lanes<RESCALE, 8>(P, graphs, graph_words, G, vals, status, s, grid_cap, wpb);
+    return launch_lod_lanes<RESCALE, 16>(P, graphs, graph_words, G, vals, status, s, grid_cap, wpb);
+}
+
 cudaError_t launch_lod(const ProblemDev& P, int precision, const uint32_t* graphs, int64_t graph_words, int G,
                        double* vals, int* status, cudaStream_t s, int grid_cap, int wpb) {
     const int64_t ntask = (int64_t)G * (P.M - 1) * P.n_lod;
-    int64_t grid = (ntask + wpb - 1) / wpb;
-    if (grid > grid_cap) grid = grid_cap;
-    if (grid < 1) grid = 1;
-    if (precision == 0) {
-        const size_t smem = (size_t)wpb * P.arena * sizeof(double);
-        {
-            cudaError_t e = ensure_smem((const void*)lod_kernel<double, false>, smem);
-            if (e != cudaSuccess) return e;
-        }
-        lod_kernel<double, false><<<(int)grid, wpb * 32, smem, s>>>(P, graphs, graph_words, G, vals, status);
-    } else if (precision == 2) {   // FP64 with per-rfunction power-of-two rescaling
-        const size_t smem = (size_t)wpb * P.arena * sizeof(double);
-        {
-            cudaError_t e = ensure_smem((const void*)lod_kernel<double, true>, smem);
-            if (e != cudaSuccess) return e;
-        }
-        lod_kernel<double, true><<<(int)grid, wpb * 32, smem, s>>>(P, graphs, graph_words, G, vals, status);
-    } else if (P.prog) {
+    if (precision == 0) return launch_lod64<false>(P, graphs, graph_words, G, vals, status, s, grid_cap, wpb);
+    if (precision == 2) return launch_lod64<true>(P, graphs, graph_words, G, vals, status, s, grid_cap, wpb);
+    if (P.prog) {
         const int S = P.prog_threads;
         const size_t smem = (size_t)S * P.prog_slots * sizeof(float);
         {
@@ -4760,12 +4791,15 @@ cudaError_t launch_lod(const ProblemDev& P, int precision, const uint32_t* graph
         if (pgrid > grid_cap * 4) pgrid = grid_cap * 4;
         lod_prog_kernel<<<(int)pgrid, S, smem, s>>>(P, graphs, graph_words, G, vals, status);
     } else {
-        const size_t smem = (size_t)wpb * P.arena * sizeof(float);
+        const size_t smem = (size_t)wpb * (P.arena + 16) * sizeof(float);
         {
-            cudaError_t e = ensure_smem((const void*)lod_kernel<float, true>, smem);
+            cudaError_t e = ensure_smem((const void*)lod_kernel<float, true, 32>, smem);
             if (e != cudaSuccess) return e;
         }
-        lod_kernel<float, true><<<(int)grid, wpb * 32, smem, s>>>(P, graphs, graph_words, G, vals, status);
+        int64_t grid = (ntask + wpb - 1) / wpb;
+        if (grid > grid_cap) grid = grid_cap;
+        if (grid < 1) grid = 1;
+        lod_kernel<float, true, 32><<<(int)grid, wpb * 32, smem, s>>>(P, graphs, graph_words, G, vals, status);
     }
     return cudaGetLastError();
 }
