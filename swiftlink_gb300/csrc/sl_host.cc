@@ -885,22 +885,19 @@ static std::vector<uint32_t> meiosis_relatives(const sl_problem_desc* d) {
 //          parent's alleles fixed by them too where i is heterozygous, tells
 //          the moving allele's colour: it cannot be both a's and b's.
 // Both hold when the graph as it is is legal; the sweep evaluates the rest.
-// planes: [N][words] bits over the loci.
-static std::vector<uint32_t> meiosis_flips(const sl_problem_desc* d, const std::vector<uint8_t>& geno, int words) {
+// g: genotype_planes.
+static std::vector<uint32_t> meiosis_flips(const sl_problem_desc* d, const std::vector<uint32_t>& g, int words) {
     const int N = d->n_members, F = d->n_founders;
     const size_t W = words;
     std::vector<uint32_t> hom_a(N * W), hom_b(N * W), het(N * W), below(N * W);
-    {
-        const std::vector<uint32_t> g = genotype_planes(N, d->n_markers, geno, words);
-        for (int i = 0; i < N; ++i)
-            for (size_t w = 0; w < W; ++w) {
-                const uint32_t c0 = g[2 * i * W + w], c1 = g[(2 * i + 1) * W + w];
-                hom_a[i * W + w] = c1 & ~c0;
-                hom_b[i * W + w] = c1 & c0;
-                het[i * W + w] = c0 & ~c1;
-                below[i * W + w] = c0 | c1;   // i typed; its descendants are added next
-            }
-    }
+    for (int i = 0; i < N; ++i)
+        for (size_t w = 0; w < W; ++w) {
+            const uint32_t c0 = g[2 * i * W + w], c1 = g[(2 * i + 1) * W + w];
+            hom_a[i * W + w] = c1 & ~c0;
+            hom_b[i * W + w] = c1 & c0;
+            het[i * W + w] = c0 & ~c1;
+            below[i * W + w] = c0 | c1;   // i typed; its descendants are added next
+        }
     std::vector<std::vector<int>> kids(N);
     for (int i = F; i < N; ++i) {
         kids[d->mother[i]].push_back(i);
@@ -1777,9 +1774,9 @@ int sl_create(const sl_problem_desc* d, const sl_options* opt, sl_ctx** out) {
     P.mflip = nullptr;
     P.mflip_words = (M + 31) / 32;
     if (P.ls_fast) {
-        const std::vector<uint32_t> mf = meiosis_flips(d, geno, P.mflip_words);
-        if ((rc = upload(ctx, (uint32_t**)&P.mflip, mf.data(), mf.size()))) return bail(rc);
         const std::vector<uint32_t> gp = genotype_planes(N, M, geno, P.mflip_words);
+        const std::vector<uint32_t> mf = meiosis_flips(d, gp, P.mflip_words);
+        if ((rc = upload(ctx, (uint32_t**)&P.mflip, mf.data(), mf.size()))) return bail(rc);
         if ((rc = upload(ctx, (uint32_t**)&P.gplane, gp.data(), gp.size()))) return bail(rc);
         const std::vector<uint32_t> mr = meiosis_relatives(d);
         if ((rc = upload(ctx, (uint32_t**)&P.mrel, mr.data(), mr.size()))) return bail(rc);
@@ -2448,7 +2445,7 @@ int sl_problem_meiosis_flips(const sl_problem_desc* d, const int32_t* dg, uint8_
     const int N = d->n_members, F = d->n_founders, M = d->n_markers, nm = 2 * (N - F), words = (M + 31) / 32;
     std::vector<uint8_t> geno((size_t)M * N);
     for (size_t i = 0; i < geno.size(); ++i) geno[i] = d->typed[i % N] ? d->genotypes[i] & 3 : 0;
-    const std::vector<uint32_t> mf = meiosis_flips(d, geno, words), gp = genotype_planes(N, M, geno, words);
+    const std::vector<uint32_t> gp = genotype_planes(N, M, geno, words), mf = meiosis_flips(d, gp, words);
     const std::vector<uint32_t> mr = meiosis_relatives(d);
     for (int w = 0; w < words; ++w) {
         const int n = std::min(32, M - 32 * w);
