@@ -1940,7 +1940,8 @@ __device__ __forceinline__ float fagw_like(const ProblemDev& P, const FagwTables
     // creation), copied to shared memory in 16-byte asynchronous copies that
     // complete while the founder alleles are propagated
     const bool wreg = P.W <= G;
-    const uint32_t cw = wreg && gl < P.W ? col[gl] : 0u;
+    const uint32_t toggled = 1u << (flip & 31);   // of word flip >> 5; none where flip is -1
+    const uint32_t cw = wreg && gl < P.W ? col[gl] ^ (gl == flip >> 5 ? toggled : 0u) : 0u;
     const int t0 = P.typ_off[lc], ntyp = P.typ_cnt[lc], nhet = P.typ_nhet[lc];
     const float2 lfreq = P.c_lfreq[(size_t)chain * M + lc];
 #pragma unroll 1
@@ -1964,10 +1965,9 @@ __device__ __forceinline__ float fagw_like(const ProblemDev& P, const FagwTables
             const uint2 ent = act ? s_lvl[q] : make_uint2((unsigned)F, 0u);
             const int pid = (int)ent.x;
             const int b = 2 * (pid - F);
-            const uint32_t w = wreg ? grp.shfl(cw, b >> 5) : col[b >> 5];
+            const uint32_t w = wreg ? grp.shfl(cw, b >> 5) : col[b >> 5] ^ (b >> 5 == flip >> 5 ? toggled : 0u);
             if (!act) continue;
-            const int vm = (int)((w >> (b & 31)) & 1u) ^ (flip == b);
-            const int vp = (int)((w >> ((b + 1) & 31)) & 1u) ^ (flip == b + 1);
+            const int vm = (int)((w >> (b & 31)) & 1u), vp = (int)((w >> ((b + 1) & 31)) & 1u);
             e[2 * pid] = e[(ent.y & 0xffffu) + vm];
             e[2 * pid + 1] = e[(ent.y >> 16) + vp];
         }
@@ -2732,15 +2732,27 @@ size_t ffbs_scan_smem(int M) { return ffbs_scan_scratch(ffbs_scan_threads(M)) + 
 // colour by homozygous members above it, or nobody below it is typed, the
 // toggled graph has the same terms in the same places, and its likelihood is
 // the current one; where they are fixed to opposite colours and the
-// transmitted one is known, the toggled graph is impossible.  The rest (about
-// one in 14 with 5% of the genotypes missing) are listed and evaluated by the
-// block's warps (fagw_like).
+// transmitted one is known, the toggled graph is impossible.  More follows
+// from the graph as it is (P.mrel, relatives_rule).  The rest (one in 25 to 30
+// with 5% of the genotypes missing) are listed and evaluated by the block's
+// warps (fagw_like).
 //
-// Measured, a sweep of every chain: 400 members, 10,000 SNPs, 8 chains 128 ->
-// 31 ms; 120 members, 2,000 SNPs, 10 chains 5.1 -> 2.8 ms (12 us a meiosis).
-// Bound by the evaluated likelihoods (issue with 32 warps on an SM: half of a
-// 400-member step's 33 us, 40% of a 120-member step), then by waiting for the
-// block with the most of them and by the scans' serial runs.
+// A step changes one column in 600, so the likelihoods of kMswAhead steps are
+// evaluated together at the first of them, from the columns as they are then:
+// one wait for the evaluations (5 us each, however few there are) instead of
+// four, and a fuller block waits for 4 steps' sum instead of each step's most.
+// Where a column has changed since, a step decides the locus anew and, if need
+// be, evaluates it itself (one step in two to four of the whole cluster).
+//
+// Measured, a sweep of every chain, as launches per meiosis, by a cluster, with
+// the steps evaluated together: 400 members, 10,000 SNPs, 8 chains 128 | 24.2 |
+// 23.0 ms; 120 members, 2,000 SNPs, 10 chains 5.1 | 2.66 | 2.16 ms (11 us a
+// meiosis), one chain 2.08 | 1.86; 30 members, 200 SNPs 0.39 | 0.335.  (400
+// members, 16 chains and more, in clusters of 4 or 8 blocks, whose bulk hid
+// the evaluations already: 35.9 | 37.3.)  Bound by the evaluated likelihoods
+// (issue with 32 warps on an SM: 23,000 of a 400-member step's 60,000 cycles;
+// 4,800 of 25,000 for 120 members), by waiting for the block with the most of
+// them (13,000; 5,600) and by the scans' serial runs and barriers.
 // ---------------------------------------------------------------------------
 struct MswShape {
     int cs;        // blocks per cluster
@@ -2752,10 +2764,21 @@ struct MswShape {
     size_t task, xch, loci, cols, bytes;   // shared offsets: tasks' scratch, exchange, per-locus arrays, columns; all bytes
 };
 
+// Steps whose likelihoods are evaluated together, a locus's index and step
+// among them in 16 bits, and how many likelihoods a block keeps (what does not
+// fit is evaluated at its step; one locus in 25 is evaluated at a step, so 4
+// steps fill 16% of nl).  3 or 5 steps measured within 2% of 4, 8 steps 5% slower.
+constexpr int kMswAhead = 4, kMswStepShift = 13;
+__host__ __device__ constexpr int msw_kept(int nl) { return nl / 4; }
+
 // per-locus arrays of a block: filter pairs (8), current and toggled
-// likelihood, theta (one more) and draw index (4 each), two steps' flip masks,
-// the list of loci to evaluate (2) and the decision maps (1)
-static size_t msw_locus_bytes(int nl) { return al16((size_t)nl * (8 + 4 * 4 + 2 + 1) + 4 + 16 * (size_t)(nl / 32)); }
+// likelihood, theta (one more) and draw index (4 each), what was evaluated
+// ahead (6 for each that is kept), masks (five for each step ahead, and the
+// columns changed), the list of loci to evaluate (2) and the decision maps (1)
+static size_t msw_locus_bytes(int nl) {
+    return al16((size_t)nl * (8 + 4 * 4 + 2 + 1) + 4 + (size_t)msw_kept(nl) * 6 +
+                4 * (size_t)(5 * kMswAhead + 1) * (nl / 32));
+}
 
 // Shared memory a block of msweep_kernel may take.
 constexpr size_t kMswSmem = 200 * 1024;
@@ -2783,7 +2806,7 @@ static bool msw_shape(const ProblemDev& P, int G, int eb, int cs, MswShape* out)
         s.staged = s.bytes <= kMswSmem;   // else the columns stay in global memory
         if (!s.staged) s.bytes = s.cols;
         *out = s;
-        if (s.bytes <= kMswSmem) return true;
+        if (s.bytes <= kMswSmem && s.nl <= 1 << kMswStepShift) return true;
     }
     return false;
 }
@@ -2833,36 +2856,30 @@ __global__ void __launch_bounds__(kMswThreads, 1) msweep_kernel(ProblemDev P, Ms
     float4* wmat = (float4*)(smem + sh.xch);   // every virtual warp's filter product
     int* wcnt = (int*)(wmat + 32);             // its draws (bit 30: an impossible pair somewhere in its block)
     int* wmap = wcnt + 32;                     // its decision map
-    int* ctl = wmap + 32;                      // [0, 1] loci to evaluate at even and odd steps, [2] impossible pair
+    int* ctl = wmap + 32;                      // [0, 1] loci to evaluate at even and odd steps, [2] impossible pair,
+                                               // [3] likelihoods to evaluate ahead
     float2* pr = (float2*)(smem + sh.loci);    // [nl] the step's pair, then the filtered pair
     float* cur = (float*)(pr + sh.nl);         // [nl] log2 likelihood of the column
     float* tog = cur + sh.nl;                  // [nl] with the meiosis toggled
     float* th = tog + sh.nl;                   // [nl + 1] theta to the locus below
     int* didx = (int*)(th + sh.nl + 1);        // [nl] draws above the locus in its block's run
-    uint32_t* msk = (uint32_t*)(didx + sh.nl);   // [2][2][nl / 32] flip masks of this step and the next
-    uint16_t* list = (uint16_t*)(msk + 4 * (sh.nl / 32));
+    const int nmw = sh.nl / 32, MW = P.mflip_words, kept = msw_kept(sh.nl);
+    float* eval = (float*)(didx + sh.nl);            // [kept] likelihoods evaluated ahead
+    uint32_t* msk = (uint32_t*)(eval + kept);        // [step ahead][nl / 32][5]: what the genotypes say (same, never),
+                                                     // same, to evaluate, evaluated
+    uint32_t* changed = msk + kMswAhead * 5 * nmw;   // [nl / 32] columns changed since the evaluation ahead
+    uint16_t* ahead = (uint16_t*)(changed + nmw);    // [kept] locus | step << kMswStepShift
+    uint16_t* list = ahead + kept;
     uint8_t* maps = (uint8_t*)(list + sh.nl);
     uint32_t* gcol = dg + ((size_t)chain * M + lo) * W;
     uint32_t* col = sh.staged ? (uint32_t*)(smem + sh.cols) : gcol;
     const int32_t* ord = order + cr * ostride;
-    const int nmw = sh.nl / 32, MW = P.mflip_words;
     if (sh.staged)
 #pragma unroll 1
         for (int i = tid; i < nl * W; i += NT) col[i] = gcol[i];
 #pragma unroll 1
     for (int i = tid; i <= nl; i += NT) th[i] = lo + i > 0 && lo + i < M ? P.c_theta_f[(size_t)chain * (M - 1) + lo + i - 1] : 0.f;
-    auto load_masks = [&](int step) {   // both masks of the step's meiosis into its buffer
-        if (step >= nm) return;
-        const uint32_t* src = P.mflip + (size_t)ord[step] * 2 * MW;
-        uint32_t* dst = msk + (step & 1) * 2 * nmw;
-#pragma unroll 1
-        for (int i = tid; i < 2 * nmw; i += NT) {
-            const int k = i >= nmw, w = (k ? i - nmw : i) + (lo >> 5);
-            dst[i] = w < MW ? src[k * MW + w] : 0u;
-        }
-    };
-    load_masks(0);
-    if (tid < 3) ctl[tid] = 0;
+    if (tid < 4) ctl[tid] = 0;
     __syncthreads();
     // the likelihood of every column as it is
 #pragma unroll 1
@@ -2883,58 +2900,118 @@ __global__ void __launch_bounds__(kMswThreads, 1) msweep_kernel(ProblemDev P, Ms
     const int vw = rank * sh.vpb + warp;                  // this warp's virtual warp
     const bool scans = warp < sh.vpb && vw < nw;
     const int s0 = min(M, (vw * 32 + lane) * L) - lo, s1 = min(M, (vw * 32 + lane + 1) * L) - lo;   // its run of loci
-    // the genotypes of a step's relatives at this warp's first 32 loci, read a step ahead
-    Relative next = load_relative(P, nm > 0 ? ord[0] : 0, (lo + warp * 32) >> 5, lane);
+    int na = 0;   // likelihoods evaluated ahead
+    // a meiosis at 32 loci: the loci where its toggling is known to change nothing, and those to evaluate
+    auto classify = [&](int m, int w, uint32_t of, uint32_t same, uint32_t never, auto relative, uint32_t* out_same) {
+        const int i = 32 * w + lane;
+        const bool in = i < nl;
+        const uint32_t* mine = col + (size_t)(in ? i : 32 * w) * W;
+        if (__any_sync(FULLMASK, in && ((of & ~(same | never)) >> lane) & 1))
+            flips_by_relatives(P, m, relative(), mine, (mine[m >> 5] >> (m & 31)) & 1, &same, &never);
+        *out_same = same;
+        return __ballot_sync(FULLMASK, in && (cur[in ? i : 0] == -INFINITY || !(((same | never) >> lane) & 1)));
+    };
 #pragma unroll 1
     for (int j = 0; j < nm; ++j) {
-        const int m = ord[j], mw = m >> 5, mb = m & 31;
-        // the step's pairs: from the genotypes where they decide, else listed
-        const uint32_t* em = msk + (j & 1) * 2 * nmw;
+        const int m = ord[j], mw = m >> 5, mb = m & 31, s = j % kMswAhead;
+        if (s == 0) {
+            // this step and the next ones as the columns are now; a task's genotypes are read while the one before goes on
+            const int tasks = min(kMswAhead, nm - j) * nmw;
+            uint32_t gs = 0u, gn = 0u;
+            Relative rel = {kNoRelative, 0u, 0u};
+            auto read = [&](int t) {
+                const int q = t / nmw, gw = (lo >> 5) + t - q * nmw;
+                if (t >= tasks || gw >= MW) return;
+                const int m2 = ord[j + q];
+                gs = P.mflip[(size_t)m2 * 2 * MW + gw];
+                gn = P.mflip[((size_t)m2 * 2 + 1) * MW + gw];
+                rel = load_relative(P, m2, gw, lane);
+            };
+            read(warp);
+#pragma unroll 1
+            for (int t = warp; t < tasks; t += NT >> 5) {
+                const int q = t / nmw, w = t - q * nmw;
+                if (q == 0 && lane == 0) changed[w] = 0u;
+                const uint32_t ts = gs, tn = gn;
+                const Relative tr = rel;
+                read(t + (NT >> 5));
+                if (32 * w >= nl) continue;
+                uint32_t same;
+                const uint32_t hard = classify(ord[j + q], w, FULLMASK, ts, tn, [&] { return tr; }, &same);
+                int at = 0;
+                if (lane == 0 && hard) at = atomicAdd(&ctl[3], __popc(hard));
+                at = __shfl_sync(FULLMASK, at, 0) + __popc(hard & ((1u << lane) - 1u));
+                const bool mine = (hard >> lane) & 1 && at < kept;
+                if (mine) ahead[at] = (uint16_t)((32 * w + lane) | q << kMswStepShift);
+                const uint32_t has = __ballot_sync(FULLMASK, mine);
+                if (lane < 5) msk[t * 5 + lane] = lane == 0 ? ts : lane == 1 ? tn : lane == 2 ? same : lane == 3 ? hard : has;
+            }
+            __syncthreads();
+            na = min(ctl[3], kept);
+        }
+        // the step's pairs: from the genotypes where they decide, evaluated ahead, else listed
 #pragma unroll 1
         for (int i0 = warp * 32; i0 < nl; i0 += NT) {
-            const int i = i0 + lane;
+            const int i = i0 + lane, w = i0 >> 5;
             const bool in = i < nl;
-            const float keep = in ? cur[i] : 0.f;
-            const uint32_t* mine = col + (size_t)(in ? i : i0) * W;
-            const int tb = (mine[mw] >> mb) & 1;
-            uint32_t same = em[i0 >> 5], never = em[nmw + (i0 >> 5)];
-            if (__any_sync(FULLMASK, in && !(((same | never) >> lane) & 1)))
-                flips_by_relatives(P, m, i0 == warp * 32 ? next : load_relative(P, m, (lo + i0) >> 5, lane), mine,
-                                   tb, &same, &never);
-            const bool sm = (same >> lane) & 1, nv = (never >> lane) & 1;
-            const bool hard = in && (keep == -INFINITY || !(sm || nv));
-            if (in) {
-                tog[i] = sm ? keep : -INFINITY;
-                pr[i] = sm ? make_float2(1.f, 1.f) : make_float2(tb ? 0.f : 1.f, tb ? 1.f : 0.f);
+            const uint32_t* k = msk + (s * nmw + w) * 5;
+            const uint32_t ch = changed[w];
+            uint32_t same = k[2], hard = k[3];
+            const uint32_t has = k[4] & ~ch;
+            if (ch) {
+                uint32_t sn;
+                const uint32_t hn = classify(m, w, ch, k[0], k[1], [&] { return load_relative(P, m, (lo >> 5) + w, lane); }, &sn);
+                same = (same & ~ch) | (sn & ch);
+                hard = (hard & ~ch) | (hn & ch);
             }
-            const unsigned b = __ballot_sync(FULLMASK, hard);
+            if (in) {
+                const bool sm = (same >> lane) & 1;
+                const int tb = (col[(size_t)i * W + mw] >> mb) & 1;
+                if (!((has >> lane) & 1)) {
+                    tog[i] = sm ? cur[i] : -INFINITY;
+                    pr[i] = sm ? make_float2(1.f, 1.f) : make_float2(tb ? 0.f : 1.f, tb ? 1.f : 0.f);
+                }
+            }
+            hard &= ~has;
             int at = 0;
-            if (lane == 0 && b) at = atomicAdd(&ctl[j & 1], __popc(b));
+            if (lane == 0 && hard) at = atomicAdd(&ctl[j & 1], __popc(hard));
             at = __shfl_sync(FULLMASK, at, 0);
-            if (hard) list[at + __popc(b & ((1u << lane) - 1u))] = (uint16_t)i;
+            if ((hard >> lane) & 1) list[at + __popc(hard & ((1u << lane) - 1u))] = (uint16_t)i;
         }
-        load_masks(j + 1);
-        next = load_relative(P, j + 1 < nm ? ord[j + 1] : m, (lo + warp * 32) >> 5, lane);
+        // the pair of column i whose toggled likelihood is lk
+        auto take = [&](int i, float lk) {
+            const float keep = cur[i];
+            const int tb = (col[(size_t)i * W + mw] >> mb) & 1;
+            tog[i] = lk;
+            float r2[2];
+            put_raw32_log2(r2, 0, tb ? lk : keep, tb ? keep : lk);
+            pr[i] = make_float2(r2[0], r2[1]);
+            if (keep == -INFINITY && lk == -INFINITY) {
+                ctl[2] = 1;
+                set_status(status, ST_ILLEGAL_DG);
+            }
+        };
         __syncthreads();
         const int nh = ctl[j & 1];
-        if (tid == 0) ctl[(j + 1) & 1] = 0;
+        if (tid == 0) ctl[(j + 1) & 1] = ctl[3] = 0;
+        if (s > 0)
 #pragma unroll 1
-        for (int h = warp * kLoci; h < nh; h += (NT >> 5) * kLoci) {
-            const int k = h + lane / G;
-            const bool valid = k < nh;
-            const int i = list[valid ? k : h];
-            const float lk = fagw_like<G, E>(P, tab, scratch, col + (size_t)i * W, chain, lo + i, m, status);
+            for (int e = tid; e < na; e += NT) {
+                const int a = ahead[e], i = a & ((1 << kMswStepShift) - 1);
+                if (a >> kMswStepShift == s && !((changed[i >> 5] >> (i & 31)) & 1)) take(i, eval[e]);
+            }
+        // what is to be evaluated: ahead when the step is the first of its group, then the step's own list
+        const int n0 = s == 0 ? na : 0;
+#pragma unroll 1
+        for (int h = warp * kLoci; h < n0 + nh; h += (NT >> 5) * kLoci) {
+            const bool valid = h + lane / G < n0 + nh;
+            const int k = valid ? h + lane / G : h;
+            const int e = k < n0 ? ahead[k] : list[k - n0];
+            const int i = k < n0 ? e & ((1 << kMswStepShift) - 1) : e, q = k < n0 ? e >> kMswStepShift : 0;
+            const float lk = fagw_like<G, E>(P, tab, scratch, col + (size_t)i * W, chain, lo + i, ord[j + q], status);
             if ((lane & (G - 1)) == 0 && valid) {
-                const float keep = cur[i];
-                const int tb = (col[(size_t)i * W + mw] >> mb) & 1;
-                tog[i] = lk;
-                float r2[2];
-                put_raw32_log2(r2, 0, tb ? lk : keep, tb ? keep : lk);
-                pr[i] = make_float2(r2[0], r2[1]);
-                if (keep == -INFINITY && lk == -INFINITY) {
-                    ctl[2] = 1;
-                    set_status(status, ST_ILLEGAL_DG);
-                }
+                if (q == 0) take(i, lk);
+                else eval[k] = lk;
             }
         }
         __syncthreads();
@@ -3080,6 +3157,7 @@ __global__ void __launch_bounds__(kMswThreads, 1) msweep_kernel(ProblemDev P, Ms
                 if (sv != (int)((w >> mb) & 1u)) {
                     col[(size_t)i * W + mw] = w ^ (1u << mb);
                     cur[i] = tog[i];
+                    atomicOr(&changed[i >> 5], 1u << (i & 31));
                 }
             }
         }

@@ -141,3 +141,26 @@ def test_sweep_is_the_same_whatever_the_cluster(members, markers, untyped):
     assert not np.array_equal(got[1], dg)
     assert np.array_equal(got[1], got[5]) and np.array_equal(got[1], got[7])
     assert np.array_equal(got[8], got[40])
+
+
+# groups of steps whose likelihoods are evaluated together: whole, cut short, more of them than a block keeps (untyped
+# members), columns that change within a group
+@pytest.mark.gpu
+@pytest.mark.parametrize("members,markers,untyped,missing,steps", [
+    (25, 40, 0.0, 0.05, 1), (25, 40, 0.0, 0.05, 3), (25, 70, 0.3, 0.05, 4), (25, 70, 0.6, 0.4, 5),
+    (40, 129, 0.0, 0.7, 22), (60, 1000, 0.4, 0.2, 31)])
+@pytest.mark.parametrize("chains", [2, 8])
+def test_sweep_is_its_steps_one_by_one(members, markers, untyped, missing, steps, chains):
+    g = family(members, 1, markers, untyped, missing, members + markers)
+    nm = min(len(g["meioses"]), steps)
+    prob = api.Problem.from_arrays(g, with_legal=False)
+    u = np.random.default_rng(steps).random((chains, nm, markers))
+    dg = np.broadcast_to(np.ascontiguousarray(g["dg0"], np.int32), (chains,) + g["dg0"].shape)
+    out = []
+    for step in (nm, 1):
+        with api.Context(prob, n_chains=chains, sampler_precision=api.SL_SAMPLER_FAST) as ctx:
+            ctx.set_graphs(dg)
+            for k in range(0, nm, step):
+                ctx.msampler_sweep(g["meioses"][k:k + step], np.ascontiguousarray(u[:, k:k + step]), n_chains=chains)
+            out.append(ctx.get_graphs())
+    assert np.array_equal(out[0], out[1])
