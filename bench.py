@@ -359,12 +359,13 @@ def issue_estimate(C, it0, it1, seed, lprob, n_meioses, sm_mhz, sms, seconds, co
     of the L- and M-sweeps they ran (each chain's L/M choice replayed with the
     same Philox draws; instructions per unit from ncu counts of the same
     workload: one chain's L half-sweep with the lane group in use, one chain's
-    meiosis step in the founder-allele-graph and filter kernels) over the SMs'
+    M-sweep, or its meiosis step in the founder-allele-graph and filter
+    kernels where the sweep runs as those) over the SMs'
     issue rate (4 schedulers per SM, one warp instruction per cycle each, at
     the SM clock sampled during the launches).  The scoring launches are left
     out.  With `shares` (each class's share of a profiled pass's kernel time)
     each class's instructions are also set against its share of the time."""
-    need = ("fag_per_meiosis_step", "scan_per_meiosis_step")
+    need = ("fag_per_meiosis_step", "scan_per_meiosis_step") if "m_sweep_per_chain" not in (counts or {}) else ()
     if not counts or any(counts.get(k) is None for k in need) or not sm_mhz or not sms or seconds <= 0:
         return None
     per_half = counts.get("l_half_sweep_per_chain")
@@ -375,7 +376,9 @@ def issue_estimate(C, it0, it1, seed, lprob, n_meioses, sm_mhz, sms, seconds, co
     n_l = int(lm_choices(C, it0, it1, seed, lprob).sum())
     n_m = C * (it1 - it0) - n_l
     per_l = 2 * per_half
-    per_m = (n_meioses + 1) * counts["fag_per_meiosis_step"] + n_meioses * counts["scan_per_meiosis_step"]
+    per_m = counts.get("m_sweep_per_chain")
+    if per_m is None:
+        per_m = (n_meioses + 1) * counts["fag_per_meiosis_step"] + n_meioses * counts["scan_per_meiosis_step"]
     inst = n_l * per_l + n_m * per_m
     peak = sms * 4 * sm_mhz * 1e6
     out = {"bound": "issue", "achieved": inst / seconds / 1e9, "peak": peak / 1e9, "unit": "G warp-inst/s",
@@ -493,13 +496,13 @@ def run_ours(args):
     per_locus = -(-N // 4) + 2 * (-(-(N - F) // 4)) + 8
     sb = step_bytes(N, F, M)
     classes = {
-        0: ("lsampler_kernel<float> (one half-sweep of the chains that chose L)",
+        0: ("lsampler_quad_kernel<float> (one half-sweep of the chains that chose L)",
             float(n_l.sum()) * (M // 2) * per_locus / max(1, kern[0][1])),
-        1: ("M-sweep graph (fag_warp_kernel + ffbs_scan_kernel, every meiosis of the chains that chose M)",
+        1: ("msweep_kernel (the M-sweep of the chains that chose M)",
             float((C - n_l).sum()) * sb / max(1, kern[1][1])),
     }
     tot = max(1e-9, sum(x[0] for x in kern.values()))
-    names = {0: "lsampler_kernel", 1: "fag_warp_kernel+ffbs_scan_kernel", 2: "LOD scoring kernel",
+    names = {0: "lsampler_quad_kernel", 1: "msweep_kernel", 2: "LOD scoring kernel",
              3: "lod_merge_kernel", 4: "choose/shuffle"}
     dom = 0 if kern[0][0] >= kern[1][0] else 1
     dom_name, dom_bytes = classes[dom]
@@ -509,7 +512,7 @@ def run_ours(args):
     peak = float(peaks.get("hbm_gbs", 6800.0))
     achieved = dom_bytes / dom_s / 1e9
     cnt = counters()
-    ck = cnt.get("lsampler_kernel_cfg5" if dom == 0 else "msweep_cfg5", {})
+    ck = cnt.get("lsampler_quad_kernel_cfg5" if dom == 0 else "msweep_cfg5", {})
     traffic = None
     if ck.get("dram_bytes_per_unit") is not None:
         units = float(n_l.sum()) * (M // 2) / max(1, kern[0][1]) if dom == 0 else \
@@ -625,11 +628,12 @@ def run_ours(args):
                "lod_positions_per_s": lod_pos_s * world,
                "lod_kernel": {"selected": int(lsel), "specialised_compile_ms": round(ljit_ms, 1),
                               "selection": "timed at the first scoring (SL_LOD_KERNEL_AUTO)"},
-               "ls_kernel": {"selected": "lsampler_kernel<float> (compact rfunctions)", "lanes": ls_lanes,
+               "ls_kernel": {"selected": ("lsampler_quad_kernel<float>" if ls_lanes == 4 else "lsampler_kernel<float>")
+                             + " (compact rfunctions)", "lanes": ls_lanes,
                              "timed_half_sweep_ms": {"32": round(ls_t[0], 3), "16": round(ls_t[1], 3),
                                                      "8": round(ls_t[2], 3)},
-                             "selection": "SL_LS_KERNEL_GENERIC: 32, 16 or 8 lanes per (chain, locus) task, "
-                                          "timed before the first sweep"},
+                             "selection": "SL_LS_KERNEL_GENERIC: 4 lanes per (chain, locus) task where its operations "
+                                          "and arena suit it, else 32, 16 or 8, timed before the first sweep"},
                "plain": {"steps_per_s": plain_steps_s * world, "lod_positions_per_s": plain_lod_pos_s * world,
                          "form": "one chain per launch, exact FP64 samplers, FP64 LOD peel with rescaling",
                          "plain_fp64_positions_underflowed": plain_underflow},

@@ -1978,7 +1978,7 @@ int sl_create(const sl_problem_desc* d, const sl_options* opt, sl_ctx** out) {
             req != SL_LS_KERNEL_AUTO && req != SL_LS_KERNEL_GENERIC32 && req != SL_LS_KERNEL_GENERIC16 &&
             req != SL_LS_KERNEL_GENERIC8 && req != SL_LS_KERNEL_GENERIC4)
             return bail(fail(nullptr, SL_EINVAL, "unknown ls_kernel %d", req));
-        if (req == SL_LS_KERNEL_GENERIC) ctx->ls_tune_pending = true;   // 32, 16 or 8 lanes per task, by timing
+        if (req == SL_LS_KERNEL_GENERIC) ctx->ls_tune_pending = true;   // 4 lanes per task by rule, else 32, 16 or 8 by timing
         if (req == SL_LS_KERNEL_GENERIC16) ctx->ls_choice = LS_GEN16;
         if (req == SL_LS_KERNEL_GENERIC8) ctx->ls_choice = LS_GEN8;
         if (req == SL_LS_KERNEL_GENERIC4) {
