@@ -2746,10 +2746,10 @@ size_t ffbs_scan_smem(int M) { return ffbs_scan_scratch(ffbs_scan_threads(M)) + 
 //
 // Measured, a sweep of every chain, as launches per meiosis, by a cluster, with
 // the steps evaluated together: 400 members, 10,000 SNPs, 8 chains 128 | 24.2 |
-// 23.0 ms; 120 members, 2,000 SNPs, 10 chains 5.1 | 2.66 | 2.16 ms (11 us a
+// 23.0 ms (19.8 in clusters of 11 blocks, msw_choose); 120 members, 2,000 SNPs, 10 chains 5.1 | 2.66 | 2.16 ms (11 us a
 // meiosis), one chain 2.08 | 1.86; 30 members, 200 SNPs 0.39 | 0.335.  (400
-// members, 16 chains and more, in clusters of 4 or 8 blocks, whose bulk hid
-// the evaluations already: 35.9 | 37.3.)  Bound by the evaluated likelihoods
+// members, 32 chains, in clusters of 4 blocks, whose bulk hid the evaluations
+// already: 35.9 | 37.3.)  Bound by the evaluated likelihoods
 // (issue with 32 warps on an SM: 23,000 of a 400-member step's 60,000 cycles;
 // 4,800 of 25,000 for 120 members), by waiting for the block with the most of
 // them (13,000; 5,600) and by the scans' serial runs and barriers.
@@ -4623,18 +4623,25 @@ static bool msw_fits(const ProblemDev& P, int G, int eb) {
     return P.mflip && 2 * P.F < 8192 && msw_shape(P, G, eb, 16, &sh);
 }
 
-// The most blocks per cluster (16, 8, 4, 2 or 1) at which `load` chains'
-// clusters are all resident, by the occupancy calculator; the fewest that fit
-// when none is.  A sweep of the 400-member, 10,000-SNP pedigree took 20.4,
-// 30.8 and 48.4 ms with 16, 8 and 4 blocks for one chain, 101, 77 and 49 ms
+// The most blocks per cluster, of the sizes that give every block as many scan
+// warps (16, 11, 8, 7, 6, 5, 4, 3, 2, 1 for 32 scan warps), at which `load`
+// chains' clusters are all resident, by the occupancy calculator; the fewest
+// that fit when none is.  A sweep of the 400-member, 10,000-SNP pedigree took
+// 20.4, 30.8 and 48.4 ms with 16, 8 and 4 blocks for one chain, 101, 77 and 49 ms
 // for 32 chains; of the 120-member one 2.2, 2.4 and 3.2 ms for one, 31, 15 and
-// 7.8 ms (6.7 with 2 blocks) for 80 chains.
+// 7.8 ms (6.7 with 2 blocks) for 80 chains (before likelihoods were evaluated
+// ahead).  With the sizes between the powers of two: 400 members, 8 chains (11
+// blocks instead of 8) 23.0 -> 19.8 ms, 16 chains 37.4 -> 29.5, 24 chains 37.4 ->
+// 32.7; 120 members, 40 chains 3.64 -> 3.05, 16 chains 2.65 -> 2.53.
 static cudaError_t msw_choose(const ProblemDev& P, int G, int eb, int load, MswShape* out) {
     const void* mk = msw_kernel(G, eb);
     cudaError_t e = cudaFuncSetAttribute(mk, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    for (int cs = 16; cs >= 1 && e == cudaSuccess; cs /= 2) {
+    int last = 0;
+    for (int cs = 16; cs >= 1 && e == cudaSuccess; --cs) {
         MswShape sh;
         if (!msw_shape(P, G, eb, cs, &sh)) break;
+        if (sh.cs == last) continue;   // as many scan warps a block as the size before
+        last = sh.cs;
         *out = sh;
         if ((e = ensure_smem(mk, sh.bytes)) != cudaSuccess) break;
         cudaLaunchConfig_t cfg;

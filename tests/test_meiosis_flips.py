@@ -164,3 +164,22 @@ def test_sweep_is_its_steps_one_by_one(members, markers, untyped, missing, steps
                 ctx.msampler_sweep(g["meioses"][k:k + step], np.ascontiguousarray(u[:, k:k + step]), n_chains=chains)
             out.append(ctx.get_graphs())
     assert np.array_equal(out[0], out[1])
+
+
+# clusters of every size between 16 and 1 blocks, as the number of chains shapes them, and scan warps that a size does not divide
+@pytest.mark.gpu
+@pytest.mark.parametrize("members,markers", [(30, 200), (60, 1000), (110, 2113)])
+def test_sweep_is_the_same_in_clusters_of_any_size(members, markers):
+    g = family(members, 1, markers, 0.1, 0.05, members)
+    prob = api.Problem.from_arrays(g, with_legal=False)
+    u = np.random.default_rng(4).random((6, markers))
+    dg = np.ascontiguousarray(g["dg0"], np.int32)
+    got = []
+    for chains in (8, 9, 13, 16, 20, 28, 36, 48, 70, 160):
+        with api.Context(prob, n_chains=chains, sampler_precision=api.SL_SAMPLER_FAST) as ctx:
+            ctx.set_graphs(np.broadcast_to(dg, (chains,) + dg.shape))
+            ctx.msampler_sweep(g["meioses"][:6], np.broadcast_to(u, (chains,) + u.shape), n_chains=chains)
+            out = ctx.get_graphs()
+        assert all(np.array_equal(out[0], x) for x in out), f"{chains} chains: a chain differs from the first"
+        got.append(out[0])
+    assert all(np.array_equal(got[0], x) for x in got)
