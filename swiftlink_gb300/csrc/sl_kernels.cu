@@ -2265,14 +2265,16 @@ __device__ void ffbs_serial_chain(const ProblemDev& P, uint32_t* G, int chain, i
 // a y > 0.  So a run of loci from one such locus to the next is filtered by
 // itself, the same operations on the same values, and the runs side by side: a
 // warp's lanes each take the run that starts at their locus.  That holds while
-// no product underflows; loci whose larger likelihood, or whose smaller
-// non-zero filtered value, lies below kExactTiny set the chain's flag, and
+// no product underflows, in the filter or in the sampling (which draws where
+// both of a locus's values are non-zero, one of them times theta): loci whose
+// larger likelihood, or whose smaller non-zero filtered value, lies below
+// kExactTiny, and any theta below kExactTheta, set the chain's flag, and
 // ffbs_exact_kernel then does it all in one run.  The serial recursion is
 // bound by the latency of FP64 (about 900 cycles a locus, two divisions and
 // five dependent operations): an M-sweep of two chains of 30 members took 13.7
 // ms at 200 SNPs and 121 ms at 2,000, in runs 2.6 and 3.6 ms; one of 120
 // members and 2,000 SNPs 549 and 36 ms.
-constexpr double kExactTiny = 1e-280;
+constexpr double kExactTiny = 1e-280, kExactTheta = 1e-20;
 
 __global__ void __launch_bounds__(32) ffbs_exact_runs_kernel(ProblemDev P, int first, int nchain, const uint8_t* sel,
                                                              int want, const uint8_t* badc, const double* raw64,
@@ -2295,10 +2297,10 @@ __global__ void __launch_bounds__(32) ffbs_exact_runs_kernel(ProblemDev P, int f
         if (k > 0 && k == i) {
             f0 = a0 == 0.0 ? 0.0 : 1.0;
             f1 = a0 == 0.0 ? 1.0 : 0.0;
-            tiny |= !(th[k - 1] >= 1e-20);
         } else {
             exact_filter(a0, a1, k > 0 ? th[k - 1] : 0.0, k == 0, f0, f1);
         }
+        tiny |= k > 0 && !(th[k - 1] >= kExactTheta);
         tiny |= (f0 != 0.0 && !(f0 >= kExactTiny)) || (f1 != 0.0 && !(f1 >= kExactTiny));
         fb[2 * k] = f0;
         fb[2 * k + 1] = f1;
