@@ -46,6 +46,7 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <float.h>
+#include <limits.h>
 #include <stdint.h>
 
 #include <algorithm>
@@ -4832,14 +4833,33 @@ cudaError_t launch_msampler(const ProblemDev& P, uint32_t* dg, int first, int nc
 
 size_t fag_smem(int N, int F, int threads, int fast) { return fag_block_bytes(N, F, threads, fast); }
 
+// Warps a block of the FP64 scorer takes, of 1 to 4: as many as leave the most
+// warps resident with `warp` shared bytes each (28: what their registers allow).
+// A grid that was sized for one lane count and blocks cut to 100 KB left one
+// warp on an SM where three fit: 4,336 cells, 32 lanes 4.06 -> 1.87 ms, 10,220
+// cells 30 -> 15.
+constexpr size_t kLodBlock = 227 * 1024, kLodSM = 228 * 1024;
+static int lod64_warps(size_t warp) {
+    int best = 1;
+    size_t most = 0;
+    for (int w = 4; w >= 1; --w) {
+        if (w * warp > kLodBlock) continue;
+        const size_t resident = std::min<size_t>(28, w * (kLodSM / (w * warp + 1024)));
+        if (resident > most) {
+            most = resident;
+            best = w;
+        }
+    }
+    return best;
+}
+
 template <bool RESCALE, int L>
 static cudaError_t launch_lod_lanes(const ProblemDev& P, const uint32_t* graphs, int64_t graph_words, int G,
-                                    double* vals, int* status, cudaStream_t s, int grid_cap, int wpb) {
+                                    double* vals, int* status, cudaStream_t s) {
     const int64_t ntask = (int64_t)G * (P.M - 1) * P.n_lod;
     const size_t warp = (size_t)(32 / L) * (P.arena + 16) * sizeof(double);
-    wpb = (int)std::max<size_t>(1, std::min<size_t>(wpb, 100 * 1024 / warp));
-    const int per = wpb * (32 / L);
-    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(grid_cap, (ntask + per - 1) / per));
+    const int wpb = lod64_warps(warp), per = wpb * (32 / L);
+    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(INT_MAX, (ntask + per - 1) / per));
     const void* k = (const void*)lod_kernel<double, RESCALE, L>;
     const cudaError_t e = ensure_smem(k, wpb * warp);
     if (e != cudaSuccess) return e;
@@ -4847,26 +4867,37 @@ static cudaError_t launch_lod_lanes(const ProblemDev& P, const uint32_t* graphs,
     return cudaGetLastError();
 }
 
-// 16 lanes to a position, and 8 from 20,000 positions (128 to an SM, more than
-// the warps of 4 that are resident there): at 8 the FP64 pipe gives its whole
-// rate to fewer idle lanes, but a position takes half as long again.  16 | 8
-// lanes, plain form, 45 members: 1,000 positions 0.114 | 0.181 ms, 8,000 0.254 |
-// 0.274, 40,000 1.17 | 1.06; rescaled, 120 members: 5,000 0.94 | 1.00, 40,000
-// 6.4 | 5.7.  32 and 4 lanes are slower at every one of these but 40,000 of the
-// 45-member pedigree, where 4 measured as 8.
+// Lanes to a position: by the arena (P.arena cells), which bounds the positions on
+// an SM, and which grows with the widest cutset, whose cells more lanes share.
+//  * up to 600 cells, 16 lanes, and 8 from 20,000 positions (128 to an SM, more
+//    than the warps of 4 that are resident there): at 8 the FP64 pipe gives its
+//    whole rate to fewer idle lanes, but a position takes half as long again.
+//    32 | 16 | 8 lanes, plain form, 45 members, 156 cells: 2,000 positions 0.162 |
+//    0.129 | 0.177 ms, 8,000 0.465 | 0.252 | 0.272, 40,000 2.14 | 1.13 | 1.05; 528
+//    cells (120 members, rescaled) 0.69 | 0.53 | 0.73, 2.28 | 1.58 | 1.77, 10.5 |
+//    5.96 | 5.69;
+//  * up to 1,000, 16: 672 cells (45 members, 4 loops) 0.353 | 0.374 | 0.594, 1.14 |
+//    1.26 | 1.31, 5.24 | 4.59 | 5.06; 788 cells (120 members, 4 loops, rescaled)
+//    0.73 | 0.59 | 0.83, 2.41 | 1.69 | 1.83, 11.1 | 7.5 | 8.0;
+//  * above, 32, which every arena that a context accepts leaves room for (8 need
+//    four arenas in a warp, 16 two): 1,088 cells 0.44 | 0.55 | 0.99, 1.48 | 1.76 |
+//    2.94, 6.6 | 6.7 | 10.8 (1,256 cells of 120 members 0.93 | 0.99 | 1.54, 16.1 |
+//    13.8 | 21.0 at 40,000); 2,216 cells 12.6 | 18.9 | 34.5; 4,336 cells 27.5 | 49.1
+//    | 147; 8,784 cells 139 | 413, 8 do not fit; 15,728 cells 490, 16 do not fit.
 template <bool RESCALE>
 static cudaError_t launch_lod64(const ProblemDev& P, const uint32_t* graphs, int64_t graph_words, int G, double* vals,
-                                int* status, cudaStream_t s, int grid_cap, int wpb) {
-    if ((int64_t)G * (P.M - 1) * P.n_lod >= 20000)
-        return launch_lod_lanes<RESCALE, 8>(P, graphs, graph_words, G, vals, status, s, grid_cap, wpb);
-    return launch_lod_lanes<RESCALE, 16>(P, graphs, graph_words, G, vals, status, s, grid_cap, wpb);
+                                int* status, cudaStream_t s) {
+    if (P.arena > 1000) return launch_lod_lanes<RESCALE, 32>(P, graphs, graph_words, G, vals, status, s);
+    if (P.arena <= 600 && (int64_t)G * (P.M - 1) * P.n_lod >= 20000)
+        return launch_lod_lanes<RESCALE, 8>(P, graphs, graph_words, G, vals, status, s);
+    return launch_lod_lanes<RESCALE, 16>(P, graphs, graph_words, G, vals, status, s);
 }
 
 cudaError_t launch_lod(const ProblemDev& P, int precision, const uint32_t* graphs, int64_t graph_words, int G,
                        double* vals, int* status, cudaStream_t s, int grid_cap, int wpb) {
     const int64_t ntask = (int64_t)G * (P.M - 1) * P.n_lod;
-    if (precision == 0) return launch_lod64<false>(P, graphs, graph_words, G, vals, status, s, grid_cap, wpb);
-    if (precision == 2) return launch_lod64<true>(P, graphs, graph_words, G, vals, status, s, grid_cap, wpb);
+    if (precision == 0) return launch_lod64<false>(P, graphs, graph_words, G, vals, status, s);
+    if (precision == 2) return launch_lod64<true>(P, graphs, graph_words, G, vals, status, s);
     if (P.prog) {
         const int S = P.prog_threads;
         const size_t smem = (size_t)S * P.prog_slots * sizeof(float);
