@@ -1958,7 +1958,7 @@ int sl_create(const sl_problem_desc* d, const sl_options* opt, sl_ctx** out) {
             // the two forms compile concurrently (NVRTC programs are independent)
             std::thread th([&] {
                 cudaSetDevice(ctx->device);
-                if (req != SL_LOD_KERNEL_JIT_SMEM) rc_reg = jit_lod_compile(in, jit_lod_threads(prog.slots), false, &ctx->jit_reg, &log_reg);
+                if (req != SL_LOD_KERNEL_JIT_SMEM) rc_reg = jit_lod_compile(in, kJitLodThreads, false, &ctx->jit_reg, &log_reg);
             });
             if (req != SL_LOD_KERNEL_JIT_REG && S)
                 rc_smem = jit_lod_compile(in, S, true, &ctx->jit_smem, &log_smem);

@@ -72,17 +72,24 @@ std::string jit_source(const JitProgramIn& in, int threads, bool shared) {
     emitf(s, "#define S %d\n", threads);
     s += "typedef unsigned int u32;\n"
          "#ifdef __CUDA_ARCH__\n#define TOGETHER() __syncthreads()\n#else\n#define TOGETHER()\n#endif\n";
+    const bool together = jit_lod_together(in, shared);
+    // blocks an SM has to hold (a second bound of 1 is not the same as none: 35 -> 38 us, 32 graphs of 30 members)
+    const std::string bounds = together && !shared ? "S, " + std::to_string(std::max(1, 512 / threads)) : "S";
     emitf(s,
-          "extern \"C\" __global__ void __launch_bounds__(S) sl_lod_jit(const u32* __restrict__ graphs, long long gw,\n"
+          "extern \"C\" __global__ void __launch_bounds__(%s) sl_lod_jit(const u32* __restrict__ graphs, long long gw,\n"
           "    int G, double* __restrict__ vals, int* status, const float* __restrict__ partial,\n"
-          "    const double* __restrict__ lt_tab, const double* __restrict__ la_tab) {\n");
+          "    const double* __restrict__ lt_tab, const double* __restrict__ la_tab) {\n",
+          bounds.c_str());
     if (shared) s += "  extern __shared__ float sh[];\n  float* A = sh + threadIdx.x;\n";
     emitf(s, "  const long long npos = %lldLL;\n", (long long)npos);
     s += "  const long long ntask = (long long)G * npos;\n";
-    // the whole block goes through the loop together: threads past the last task repeat it and write nothing
-    s += "  for (long long t0 = (long long)blockIdx.x * S; t0 < ntask; t0 += (long long)gridDim.x * S) {\n"
-         "    const bool mine = t0 + threadIdx.x < ntask;\n"
-         "    const long long t = mine ? t0 + threadIdx.x : ntask - 1;\n";
+    // together: threads past the last task repeat it and write nothing
+    if (together)
+        s += "  for (long long t0 = (long long)blockIdx.x * S; t0 < ntask; t0 += (long long)gridDim.x * S) {\n"
+             "    const bool mine = t0 + threadIdx.x < ntask;\n"
+             "    const long long t = mine ? t0 + threadIdx.x : ntask - 1;\n";
+    else
+        s += "  for (long long t = (long long)blockIdx.x * S + threadIdx.x; t < ntask; t += (long long)gridDim.x * S) {\n";
     emitf(s, "    const int b = (int)(t / npos);\n    const int pidx = (int)(t %% npos);\n");
     emitf(s, "    const int l = pidx / %d, o = pidx %% %d;\n", in.n, in.n);
     emitf(s, "    const u32* cL = graphs + (long long)b * gw + (long long)l * %d;\n    const u32* cR = cL + %d;\n", in.W,
@@ -197,7 +204,7 @@ std::string jit_source(const JitProgramIn& in, int threads, bool shared) {
             for (int q = 0; q < cnt; ++q)
                 emitf(s, "      %s = ldexpf(%s, -e%d);\n", news[q].c_str(), olds[q].c_str(), k);
             s += "    }\n";
-            if (k % 4 == 3) s += "    TOGETHER();\n";
+            if (together && k % 4 == 3) s += "    TOGETHER();\n";
         } else {   // LI_END
             const int rs = pc[1];
             result = rs >= 0 ? ref(rs) : std::string("0.0f");
@@ -214,7 +221,7 @@ std::string jit_source(const JitProgramIn& in, int threads, bool shared) {
           "    else v = (double)logf(result) + (double)scale * 0.69314718055994530942 - rec - (%.17g);\n",
           in.zero_ok ? "" : ("atomicCAS(status, 0, " + std::to_string((int)ST_LOD_NONPOS) + ");").c_str(),
           in.marker_trans);
-    s += "    if (mine) vals[t] = v;\n  }\n}\n";
+    s += together ? "    if (mine) vals[t] = v;\n  }\n}\n" : "    vals[t] = v;\n  }\n}\n";
     return s;
 }
 

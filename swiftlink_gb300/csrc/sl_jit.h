@@ -21,13 +21,25 @@ struct JitProgramIn {
     int zero_ok;             // a zero trait likelihood is a zero term, not an error
 };
 
-// Threads per block of the scorer with its values in registers.  A block's
-// warps start together and so fetch the straight-line code together: 64 graphs
-// of the 120-member pedigree (146 slots) took 0.60 ms in blocks of 128, 0.32
-// in blocks of 512 (4 graphs 67 and 36 us).  With many slots the 128 registers
-// a thread that such a block leaves are too few: 731 slots (400 members) 0.71
-// ms in blocks of 128, 0.93 in blocks of 512.
-inline int jit_lod_threads(int slots) { return slots <= 192 ? 512 : 128; }
+// Threads per block of the scorer with its values in registers, and whether its
+// warps go through the code together.  Every warp fetches the straight-line code,
+// and from about 8,000 words of program on it no longer stays in the instruction
+// cache: there a block's warps keep together (barriers), and with up to 192 slots
+// the registers are limited so that four blocks share an SM.  Apart, with all
+// registers | together, so limited, 1, 4 and 32 graphs of 2,000 SNPs: 66 members
+// (9,002 words) 19, 20, 84 | 18, 20, 80 us; 90 members (10,808) 28, 58, 271 | 27, 29,
+// 152; 130 members (184 slots) 38, 77, 363 | 38, 40, 203 (in blocks of 512 43, 41, 206:
+// one has to wait for 16 warps).  A short program only loses: 30 members (4,154
+// words) 11, 12, 35 | 10, 11, 39 (12, 13, 46), 54 members (5,141) 13, 14, 59 | 14, 14, 59.  With many
+// slots the registers left are too few: 731 slots (400 members) 0.71 ms with all,
+// 0.93 in blocks of 512; in between, 204 to 343 slots gain as much in large calls (32
+// graphs 360 -> 207, 336 -> 221 in blocks of 512) as they lose in small ones (37 -> 42,
+// 35 -> 43) and keep theirs.  The form in shared memory: 64 graphs of 120 members
+// 0.67 | 0.48 ms.
+constexpr int kJitLodThreads = 128;
+inline bool jit_lod_together(const JitProgramIn& in, bool shared) {
+    return in.n_words >= 8000 && (shared || in.slots <= 192);
+}
 
 struct JitLod {
     void* lib = nullptr;     // cudaLibrary_t
