@@ -400,6 +400,30 @@ static bool quad_ready(sl_ctx* ctx) {
     return true;
 }
 
+// The four-lane kernel's arena for one imputation call of ntask passes at once:
+// a slice for every warp they fill (up to 32 on an SM and to kQuadArenaBytes),
+// as one chain's, since the sweeps' arena is sized for half-sweeps and a call may
+// have more passes than those loci (100 passes of 4 chains, 400 members and 40
+// loci: 33 warps' slices for 50 warps, 73 ms; 38 with a slice each).  False: by si_kernel.
+static bool si_arena(sl_ctx* ctx, int64_t ntask, ProblemDev* Q, void** arena) {
+    *arena = nullptr;
+    if (!ctx->quad_ok || quad_block_bytes(*Q, 1) > kSmemBudget) return false;
+    const size_t per = quad_arena_per_warp(*Q);
+    if (!per) return true;
+    int64_t warps = (ntask + kQuadWarpTasks - 1) / kQuadWarpTasks;
+    warps = (warps + kQuadBlockWarps - 1) / kQuadBlockWarps * kQuadBlockWarps;
+    warps = std::min<int64_t>(warps, std::min<int64_t>(32 * (int64_t)ctx->sms, (int64_t)(kQuadArenaBytes / per)));
+    if (warps < kQuadBlockWarps) return false;
+    if (cudaMalloc(arena, (size_t)warps * per) != cudaSuccess) {
+        cudaGetLastError();
+        *arena = nullptr;
+        return false;
+    }
+    Q->quad_arena = *arena;
+    Q->quad_warps = warps;
+    return true;
+}
+
 static int ls_tune(sl_ctx* ctx) {
     if (!ctx->ls_tune_pending) return SL_OK;
     ctx->ls_tune_pending = false;
@@ -2140,6 +2164,18 @@ struct StreamGuard {
     bool armed = true;
     ~StreamGuard() {
         if (armed) cudaStreamSynchronize(ctx->stream);
+    }
+};
+
+// Device memory of one call, given back when it returns (after the stream's work on it).
+struct DevBuffer {
+    sl_ctx* ctx;
+    void* p = nullptr;
+    explicit DevBuffer(sl_ctx* c) : ctx(c) {}
+    ~DevBuffer() {
+        if (!p) return;
+        cudaStreamSynchronize(ctx->stream);
+        cudaFree(p);
     }
 };
 
@@ -4078,9 +4114,12 @@ int sl_sequential_imputation(sl_ctx* ctx, int32_t first, int32_t n_chains, const
     if ((rc = dev_alloc(ctx, &d_w, (size_t)n_chains))) return rc;
     CK(cudaMemcpyAsync(ctx->d_u, draws, sizeof(double) * nu, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(d_starts, start_loci, sizeof(int32_t) * n_chains, cudaMemcpyHostToDevice, ctx->stream));
+    ProblemDev P = ctx->P;
+    DevBuffer arena(ctx);
+    const bool quad = si_arena(ctx, n_chains, &P, &arena.p);
     { Prof pf_(ctx, SL_KERNEL_LSAMPLER);
-    CK(launch_si(ctx->P, ctx->d_dg, first, n_chains, d_starts, ctx->d_u, chain_stride, 0, 0, d_w, ctx->d_status,
-                 ctx->stream, ctx->ls_wpb, 1, 0, ctx->ls_grid, quad_ready(ctx), ctx->sms)); }
+    CK(launch_si(P, ctx->d_dg, first, n_chains, d_starts, ctx->d_u, chain_stride, 0, 0, d_w, ctx->d_status,
+                 ctx->stream, ctx->ls_wpb, 1, 0, ctx->ls_grid, quad, ctx->sms)); }
     CK(cudaMemcpyAsync(weights, d_w, sizeof(double) * n_chains, cudaMemcpyDeviceToHost, ctx->stream));
     rc = sl_synchronize(ctx);
     for (void* p : {(void*)d_starts, (void*)d_w}) {
@@ -4093,7 +4132,7 @@ int sl_sequential_imputation(sl_ctx* ctx, int32_t first, int32_t n_chains, const
 int sl_sequential_imputation_run(sl_ctx* ctx, int32_t iterations, uint64_t seed, double* best_weights) {
     if (!ctx || iterations < 1) return fail(ctx, SL_EINVAL, "bad arguments");
     CK(cudaSetDevice(ctx->device));
-    const ProblemDev& P = ctx->P;
+    ProblemDev P = ctx->P;
     const int C = ctx->n_chains, M = P.M;
     const size_t words = (size_t)M * P.W;
     // passes are independent (SequentialImputation::parallel_run, sequential_imputation.cc:
@@ -4109,7 +4148,8 @@ int sl_sequential_imputation_run(sl_ctx* ctx, int32_t iterations, uint64_t seed,
     if ((rc = dev_alloc(ctx, &d_starts, (size_t)C * batch))) return rc;
     if ((rc = dev_alloc(ctx, &d_w, (size_t)C * batch))) return rc;
     if ((rc = dev_alloc(ctx, &d_best, (size_t)C))) return rc;
-    const bool quad = quad_ready(ctx);
+    DevBuffer arena(ctx);
+    const bool quad = si_arena(ctx, (int64_t)C * batch, &P, &arena.p);
     std::vector<double> lowest(C, -DBL_MAX);
     CK(cudaMemcpyAsync(d_best, lowest.data(), sizeof(double) * C, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemsetAsync(scratch, 0, sizeof(uint32_t) * words * C * batch, ctx->stream));

@@ -1267,7 +1267,7 @@ __global__ void __launch_bounds__(32 * kQuadWarps) si_quad_kernel(ProblemDev P, 
     const int warp = threadIdx.x >> 5, wpb = blockDim.x >> 5, M = P.M;
     const int64_t gw = (int64_t)blockIdx.x * wpb + warp, nw = (int64_t)gridDim.x * wpb;
     Quad<T> Q = quad_bind<T>(P, prog, smem + quad_prog_bytes(P) + warp * quad_warp_bytes<T>(P),
-                             quad_arena_slice<T>(P, first, gw));
+                             quad_arena_slice<T>(P, 0, gw));
     const int64_t ntask = (int64_t)nchain * npass;
     for (int64_t g = gw; g * kQuadTasks < ntask; g += nw) {
         const int64_t t = min(g * kQuadTasks + Q.task, ntask - 1);
@@ -4556,7 +4556,7 @@ static cudaError_t launch_si_quad(const ProblemDev& P, uint32_t* dg, int first, 
     cudaError_t e = ensure_smem((const void*)si_quad_kernel<T>, smem);
     if (e != cudaSuccess) return e;
     int64_t grid = (ntask + per - 1) / per;
-    if (quad_arena_per_warp(P)) grid = std::min(grid, nchain * (P.quad_warps / wpb));   // slots of the arena
+    if (quad_arena_per_warp(P)) grid = std::min(grid, P.quad_warps / wpb);   // slices of the call's arena
     si_quad_kernel<T><<<(int)grid, 32 * wpb, smem, s>>>(P, dg, first, nchain, starts, d, 0, weights, status, npass,
                                                         pass_stride);
     return cudaGetLastError();
