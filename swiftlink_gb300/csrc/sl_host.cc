@@ -404,10 +404,22 @@ static bool quad_ready(sl_ctx* ctx) {
 // a slice for every warp they fill (up to 32 on an SM and to kQuadArenaBytes),
 // as one chain's, since the sweeps' arena is sized for half-sweeps and a call may
 // have more passes than those loci (100 passes of 4 chains, 400 members and 40
-// loci: 33 warps' slices for 50 warps, 73 ms; 38 with a slice each).  False: by si_kernel.
+// loci: 32 warps' slices for 50 warps, 73 ms; 37 with a slice each).
+//
+// False: by si_kernel, a warp a pass.  So also where the rfunctions are wide, since
+// a warp's eight passes are at different loci and go through each operation as
+// the widest of them asks: from 16 cells an operation at the widest locus on, 32
+// in FP64, unless one pass is alone or a warp a pass would be more than the SMs
+// hold at once (12 of them, 6 in FP64).  A warp a pass | four lanes, 45 members, 1, 8, 400 and 4,000
+// passes: 15 cells, 700 loci 105, 108, 109, 344 | 73, 90, 97, 101 ms; 20 cells, 200
+// loci 32, 33, 33, 105 | 25, 33, 38, 39, in FP64 69, 73, 73, 392 | 41, 58, 66, 68; 38
+// cells, 40 loci 7.1, 7.3, 7.4, 23 | 6.5, 11, 13, 14, in FP64 15, 15, 15, 80 | 11, 19,
+// 23, 25; in FP64 30 cells, 700 loci, 1, 8 and 400 246, 260, 260 | 163, 240, 270.
 static bool si_arena(sl_ctx* ctx, int64_t ntask, ProblemDev* Q, void** arena) {
     *arena = nullptr;
     if (!ctx->quad_ok || quad_block_bytes(*Q, 1) > kSmemBudget) return false;
+    const bool wide = Q->ls_arena > (Q->ls_fast ? 16 : 32) * Q->K;
+    if (wide && ntask > 1 && ntask <= (Q->ls_fast ? 12 : 6) * (int64_t)ctx->sms) return false;
     const size_t per = quad_arena_per_warp(*Q);
     if (!per) return true;
     int64_t warps = (ntask + kQuadWarpTasks - 1) / kQuadWarpTasks;
