@@ -443,11 +443,19 @@ static int ls_tune(sl_ctx* ctx) {
     const bool quad = quad_ready(ctx);
     const bool jit = ctx->jit_ls.kern != nullptr;
     // Four lanes per task without a timing where the rfunctions are small (up
-    // to 16 cells an operation at the widest locus): fastest there in every
-    // pedigree and number of chains measured, by 1.3 to 5.5 times (see
-    // lsampler_quad_kernel); wide rfunctions may want a task's cells spread
-    // over more lanes, and are timed.
-    if (quad && !jit && P.ls_arena <= 16 * P.K) {
+    // to 10 cells an operation at the widest locus): fastest there in every
+    // pedigree and number of chains measured (see lsampler_quad_kernel).  A
+    // warp's eight tasks wait for the widest, so wider rfunctions may want a
+    // task's cells spread over more lanes, and are timed.  32 | 4 lanes, 200 to 700
+    // loci, a sweep: 4.9 cells 0.45 | 0.34 ms, 8.5 0.48 | 0.45, 12.3 0.54 | 0.57, 13.5
+    // 0.40 | 0.44, 15.4 0.43 | 0.52, 20 0.52 | 0.69 (in FP64 0.95 | 0.59, 1.04 | 0.76,
+    // 1.10 | 0.97, 0.79 | 0.77, 0.83 | 0.91, 0.94 | 1.15).  Up to 16 cells four lanes
+    // win again where a warp a task would go round (12 are resident on an SM):
+    // 13.5 cells, 400 tasks 0.41 | 0.45, 2,000 tasks 0.50 | 0.44; with fewer tasks
+    // and more cells they are not timed in FP32 (the half-sweep timed may lack the
+    // widest locus: 13.5 cells, 0.40 | 0.44, chose four).
+    const bool many = (int64_t)ctx->even.size() * ctx->n_chains > 12 * (int64_t)ctx->sms;
+    if (quad && !jit && P.ls_arena <= (many ? 16 : 10) * P.K) {
         if (ctx->ls_choice != LS_QUAD) ++ctx->ls_epoch;
         ctx->ls_choice = LS_QUAD;
         return SL_OK;
@@ -476,7 +484,7 @@ static int ls_tune(sl_ctx* ctx) {
     CK(cudaMemcpyAsync(scratch, ctx->d_dg, sizeof(uint32_t) * words, cudaMemcpyDeviceToDevice, ctx->stream));
     cudaEvent_t a = take_event(ctx), b = take_event(ctx);
     std::vector<int> cand = {LS_GEN32, LS_GEN16, LS_GEN8};
-    if (quad) cand.push_back(LS_QUAD);
+    if (quad && (many || !P.ls_fast)) cand.push_back(LS_QUAD);
     if (jit) cand.push_back(LS_JIT);
     int best = ctx->ls_choice;
     float best_ms = 0.f;
