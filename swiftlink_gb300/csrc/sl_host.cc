@@ -378,7 +378,7 @@ static std::map<std::tuple<int, int, int, int, int, bool>, int> g_ls_class;
 
 // Whether the four-lane kernel can run: its shared memory, and the global
 // arena (allocated here) with room for a half-sweep of every chain, or for as
-// many warps a chain as kQuadArenaBytes holds.
+// many warps a chain as kQuadArenaBytes holds, but one.
 template <typename T>
 static int dev_alloc(sl_ctx* ctx, T** p, size_t n);
 static bool quad_ready(sl_ctx* ctx) {
@@ -387,8 +387,8 @@ static bool quad_ready(sl_ctx* ctx) {
     const size_t per = quad_arena_per_warp(P);
     if (!per || P.quad_arena) return true;
     int64_t warps = ((int64_t)ctx->even.size() + kQuadWarpTasks - 1) / kQuadWarpTasks;
-    warps = std::min<int64_t>(warps, (int64_t)(kQuadArenaBytes / per / ctx->n_chains));
-    warps = std::max<int64_t>(1, (warps + kQuadBlockWarps - 1) / kQuadBlockWarps) * kQuadBlockWarps;
+    warps = (warps + kQuadBlockWarps - 1) / kQuadBlockWarps * kQuadBlockWarps;
+    warps = std::max<int64_t>(1, std::min<int64_t>(warps, (int64_t)(kQuadArenaBytes / per / ctx->n_chains)));
     uint8_t* a = nullptr;
     if (dev_alloc(ctx, &a, (size_t)warps * per * ctx->n_chains)) {
         cudaGetLastError();
@@ -398,6 +398,16 @@ static bool quad_ready(sl_ctx* ctx) {
     P.quad_arena = a;
     P.quad_warps = warps;
     return true;
+}
+
+// Gives the arena back where the sweeps take another kernel.
+static void quad_release(sl_ctx* ctx) {
+    ProblemDev& P = ctx->P;
+    if (!P.quad_arena || ctx->ls_choice == LS_QUAD) return;
+    cudaFree(P.quad_arena);
+    ctx->owned.erase(std::find(ctx->owned.begin(), ctx->owned.end(), P.quad_arena));
+    P.quad_arena = nullptr;
+    P.quad_warps = 0;
 }
 
 // The four-lane kernel's arena for one imputation call of ntask passes at once:
@@ -439,6 +449,10 @@ static bool si_arena(sl_ctx* ctx, int64_t ntask, ProblemDev* Q, void** arena) {
 static int ls_tune(sl_ctx* ctx) {
     if (!ctx->ls_tune_pending) return SL_OK;
     ctx->ls_tune_pending = false;
+    struct Release {
+        sl_ctx* ctx;
+        ~Release() { quad_release(ctx); }
+    } release{ctx};
     const ProblemDev& P = ctx->P;
     const bool quad = quad_ready(ctx);
     const bool jit = ctx->jit_ls.kern != nullptr;

@@ -4477,6 +4477,7 @@ static int quad_warps_per_block(const ProblemDev& P, int64_t load, int nloci, in
     const int64_t warps = load * ((nloci + kQuadTasks - 1) / kQuadTasks);
     int w = (int)std::max<int64_t>(1, std::min<int64_t>(kQuadWarps, (warps + sms - 1) / sms));
     while (w > 1 && quad_block_bytes(P, w) > 110 * 1024) --w;   // two blocks to an SM
+    if (quad_arena_per_warp(P)) w = (int)std::min<int64_t>(w, P.quad_warps);   // the arena's slices
     return w;
 }
 
