@@ -78,6 +78,7 @@ static cudaError_t ensure_smem(const void* func, size_t bytes) {
     if (bytes <= have) return cudaSuccess;
     e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e == cudaSuccess) have = bytes;
+    else cudaGetLastError();   // reported here; the next launch, perhaps another context's, asks for the last error
     return e;
 }
 
