@@ -36,6 +36,7 @@ namespace sl {
 size_t lsampler_smem_per_warp(const ProblemDev& P);
 size_t lsampler_smem_shared(const ProblemDev& P);
 int lsampler_resident_tasks(const ProblemDev& P, int wpb);
+bool lsampler_fits(const ProblemDev& P, int wpb, int lanes);
 size_t quad_arena_per_warp(const ProblemDev& P);
 size_t quad_block_bytes(const ProblemDev& P, int warps);
 cudaError_t launch_lsampler(const ProblemDev& P, uint32_t* dg, int first, int nchain, const int32_t* loci,
@@ -497,7 +498,9 @@ static int ls_tune(sl_ctx* ctx) {
     CK(cudaMemcpy(&st, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost));
     CK(cudaMemcpyAsync(scratch, ctx->d_dg, sizeof(uint32_t) * words, cudaMemcpyDeviceToDevice, ctx->stream));
     cudaEvent_t a = take_event(ctx), b = take_event(ctx);
-    std::vector<int> cand = {LS_GEN32, LS_GEN16, LS_GEN8};
+    std::vector<int> cand;   // 32 lanes' block fits, or sl_create would have refused the peel sequence
+    for (int k : {LS_GEN32, LS_GEN16, LS_GEN8})
+        if (k == LS_GEN32 || lsampler_fits(P, ctx->ls_wpb, ls_lanes(k))) cand.push_back(k);
     if (quad && (many || !P.ls_fast)) cand.push_back(LS_QUAD);
     if (jit) cand.push_back(LS_JIT);
     int best = ctx->ls_choice;

@@ -4495,6 +4495,14 @@ static cudaError_t launch_quad(const ProblemDev& P, uint32_t* dg, int first, int
     return cudaGetLastError();
 }
 
+// Whether launch_lsampler's block for `lanes` (32, 16 or 8) fits the most shared
+// memory that a block may have: two and four tasks to a warp are the least that
+// those lane groups take.
+bool lsampler_fits(const ProblemDev& P, int wpb, int lanes) {
+    const int tasks = lanes == 32 ? wpb : lanes == 16 ? 2 * std::max(1, wpb / 2) : 4 * std::max(1, wpb / 4);
+    return ls_tables_bytes(P) + tasks * lsampler_smem_per_warp(P) <= 227 * 1024;
+}
+
 // lanes = 32, 16, 8 or 4 lanes per (chain, locus) task; all draw the same graphs.
 cudaError_t launch_lsampler(const ProblemDev& P, uint32_t* dg, int first, int nchain, const int32_t* loci, int nloci,
                             const double* u, int64_t ucs, int64_t uls, uint64_t seed, uint64_t iter,
@@ -4508,14 +4516,14 @@ cudaError_t launch_lsampler(const ProblemDev& P, uint32_t* dg, int first, int nc
     }
     if (lanes == 8) {
         // four tasks per warp: a quarter of the warps per block keeps the block's shared memory
-        const int w8 = wpb > 3 ? wpb / 4 : 1;
+        const int w8 = std::max(1, wpb / 4);
         if (P.ls_fast) return launch_lsampler_g<float, 8>(P, dg, first, nchain, loci, nloci, d, sel, want, status, s,
                                                           grid_cap, w8);
         return launch_lsampler_g<double, 8>(P, dg, first, nchain, loci, nloci, d, sel, want, status, s, grid_cap, w8);
     }
     if (lanes == 16) {
         // two tasks per warp: half as many warps per block keeps the block's shared memory
-        const int w16 = wpb > 1 ? wpb / 2 : 1;
+        const int w16 = std::max(1, wpb / 2);
         if (P.ls_fast) return launch_lsampler_g<float, 16>(P, dg, first, nchain, loci, nloci, d, sel, want, status, s,
                                                            grid_cap, w16);
         return launch_lsampler_g<double, 16>(P, dg, first, nchain, loci, nloci, d, sel, want, status, s, grid_cap, w16);
