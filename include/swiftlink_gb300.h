@@ -476,6 +476,14 @@ int sl_lod_kernel_info(sl_ctx* ctx, int32_t* kernel, double* compile_ms);
  * sl_last_error).  A background compile that has ended is taken up here. */
 int sl_ls_kernel_info(sl_ctx* ctx, int32_t* kernel, double* compile_ms);
 
+/* The fast M-sampler's form from the context's next sweep or run on: AUTO runs a
+ * chain's sweep as one thread-block cluster where its share of the loci fits a
+ * block's shared memory, else as two launches per meiosis; LAUNCHES takes the
+ * latter always.  Both draw the same graphs. */
+#define SL_MSAMPLER_AUTO 0
+#define SL_MSAMPLER_LAUNCHES 1
+int sl_msampler_set_form(sl_ctx* ctx, int32_t form);
+
 /* The L-sampler autotuner's outcome: the lanes per (chain, locus) task of the
  * generic kernel in use (32, 16, 8 or 4; 0 when the specialised kernel runs)
  * and the timed half-sweep of each candidate in milliseconds, times_ms[0..3] =

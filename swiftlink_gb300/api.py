@@ -24,6 +24,7 @@ SL_LOD_ZERO_OK = 1
 SL_LS_KERNEL_GENERIC, SL_LS_KERNEL_SPECIALISED, SL_LS_KERNEL_BACKGROUND, SL_LS_KERNEL_AUTO = 0, 1, 2, 3
 SL_LS_KERNEL_GENERIC32, SL_LS_KERNEL_GENERIC16, SL_LS_KERNEL_GENERIC8, SL_LS_KERNEL_GENERIC4 = 4, 5, 6, 7
 SL_KERNEL_LSAMPLER, SL_KERNEL_MSAMPLER, SL_KERNEL_LOD, SL_KERNEL_LOD_MERGE, SL_KERNEL_OTHER = 0, 1, 2, 3, 4
+SL_MSAMPLER_AUTO, SL_MSAMPLER_LAUNCHES = 0, 1
 SL_ADJOINT_WARP, SL_ADJOINT_THREAD, SL_ADJOINT_SPECIALISED = 1, 2, 3
 SL_ADJOINT_VARIANTS = 2
 
@@ -38,7 +39,7 @@ EXPORTED = [
     "sl_chain_loglik", "sl_peel_sequence", "sl_batch_create", "sl_batch_run", "sl_batch_destroy",
     "sl_sequential_imputation", "sl_sequential_imputation_run", "sl_adjoint_memory", "sl_adjoint_info",
     "sl_adjoint_set_form", "sl_adjoint_kernel_info", "sl_problem_adjoint_source", "sl_ls_tuning",
-    "sl_problem_lod_source", "sl_problem_meiosis_flips",
+    "sl_problem_lod_source", "sl_problem_meiosis_flips", "sl_msampler_set_form",
 ]
 
 
@@ -371,6 +372,10 @@ class Context:
         self._check(lib().sl_adjoint_info(self.h, ctypes.byref(f), ctypes.byref(a), ctypes.byref(b),
                                           ctypes.byref(c)))
         return f.value, a.value, b.value, c.value
+
+    def msampler_set_form(self, form: int = SL_MSAMPLER_AUTO):
+        """Fast M-sweeps as clusters where they fit (SL_MSAMPLER_AUTO), or as launches per meiosis."""
+        self._check(lib().sl_msampler_set_form(self.h, ctypes.c_int32(form)))
 
     def adjoint_set_form(self, form: int = 0, variant: int = 0):
         """Fix the adjoint's form (SL_ADJOINT_*; for SL_ADJOINT_SPECIALISED

@@ -1835,6 +1835,7 @@ int sl_create(const sl_problem_desc* d, const sl_options* opt, sl_ctx** out) {
         if ((rc = upload(ctx, (uint16_t**)&P.typ_nhet, nhet.data(), nhet.size()))) return bail(rc);
     }
     P.mflip = nullptr;
+    P.ms_launches = 0;
     P.mflip_words = (M + 31) / 32;
     if (P.ls_fast) {
         const std::vector<uint32_t> gp = genotype_planes(N, M, geno, P.mflip_words);
@@ -3173,6 +3174,23 @@ int sl_adjoint_info(sl_ctx* ctx, int32_t* form, double* warp_ms, double* thread_
     if (warp_ms) *warp_ms = ctx->adj_form_ms[0];
     if (thread_ms) *thread_ms = ctx->adj_form_ms[1];
     if (specialised_ms) *specialised_ms = ctx->adj_form_ms[2];
+    return SL_OK;
+}
+
+int sl_msampler_set_form(sl_ctx* ctx, int32_t form) {
+    if (!ctx) return fail(ctx, SL_EINVAL, "null context");
+    if (form != SL_MSAMPLER_AUTO && form != SL_MSAMPLER_LAUNCHES)
+        return fail(ctx, SL_EINVAL, "unknown M-sampler form %d", form);
+    const int launches = form == SL_MSAMPLER_LAUNCHES;
+    if (ctx->P.ms_launches == launches) return SL_OK;
+    CK(cudaSetDevice(ctx->device));
+    ctx->P.ms_launches = launches;
+    ++ctx->ls_epoch;   // the run graphs are captured again at their next launch
+    if (ctx->ms_graph) {
+        CK(cudaStreamSynchronize(ctx->stream));
+        cudaGraphExecDestroy(ctx->ms_graph);
+        ctx->ms_graph = nullptr;
+    }
     return SL_OK;
 }
 

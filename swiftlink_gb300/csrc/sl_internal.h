@@ -68,6 +68,7 @@ struct ProblemDev {
                                          // it zero, whatever the rest of a legal graph (meiosis_flips, sl_host.cc); null
                                          // in the exact mode
     int32_t mflip_words;                 // ceil(M / 32)
+    int32_t ms_launches;                 // fast M-sweeps as launches per meiosis, though a cluster fits (sl_msampler_set_form)
     const uint32_t* gplane;              // [N][2][mflip_words]: the two bits of a member's genotype codes, a bit per locus
     const uint32_t* mrel;                // [2 Nnf meioses][kRelatives]: the meiosis's relatives (flips_by_relatives)
     const double* prior;                 // [M][4 genotype codes][4 states]

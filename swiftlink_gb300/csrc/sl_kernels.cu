@@ -4633,7 +4633,7 @@ static void msw_config(const MswShape& sh, int nchain, cudaLaunchConfig_t* cfg, 
 // some shape fits (the component counts are 13-bit fields).
 static bool msw_fits(const ProblemDev& P, int G, int eb) {
     MswShape sh;
-    return P.mflip && 2 * P.F < 8192 && msw_shape(P, G, eb, 16, &sh);
+    return P.mflip && !P.ms_launches && 2 * P.F < 8192 && msw_shape(P, G, eb, 16, &sh);
 }
 
 // The most blocks per cluster, of the sizes that give every block as many scan
