@@ -604,9 +604,10 @@ def run_ours(args):
         ctx.get_graphs(out=host_graphs)
     e2e_t = allmax(time.perf_counter() - t0)
     words = M * ((2 * (N - F) + 31) // 32)
-    e2e = {"value": Ke * S * C * world / e2e_t, "unit": UNIT, "h2d_bytes_per_step": 4 * words * C,
+    # in: the device reads the non-founders' int32 indicators from the caller's array; out: packed words
+    e2e = {"value": Ke * S * C * world / e2e_t, "unit": UNIT, "h2d_bytes_per_step": 8 * (N - F) * M * C,
            "d2h_bytes_per_step": 4 * words * C,
-           "path": f"sl_set_descent_graphs (packed on the host, pinned copy) + sl_run ({S} iterations of "
+           "path": f"sl_set_descent_graphs (packed by the device from host memory) + sl_run ({S} iterations of "
                    f"{C} chains) + sl_get_descent_graphs per step, wall clock"}
 
     extras = {}
@@ -633,7 +634,7 @@ def run_ours(args):
                              "timed_half_sweep_ms": {"32": round(ls_t[0], 3), "16": round(ls_t[1], 3),
                                                      "8": round(ls_t[2], 3)},
                              "selection": "SL_LS_KERNEL_GENERIC: 4 lanes per (chain, locus) task where its operations "
-                                          "and arena suit it, else 32, 16 or 8, timed before the first sweep"},
+                                          "and arena suit it, else 32, 16, 8 or 4, timed before the first sweep"},
                "plain": {"steps_per_s": plain_steps_s * world, "lod_positions_per_s": plain_lod_pos_s * world,
                          "form": "one chain per launch, exact FP64 samplers, FP64 LOD peel with rescaling",
                          "plain_fp64_positions_underflowed": plain_underflow},

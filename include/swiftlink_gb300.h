@@ -134,10 +134,10 @@ typedef struct sl_options {
 #define SL_LS_KERNEL_AUTO 3
 /* GENERIC gives a (chain, locus) task 4 lanes (eight tasks per warp) where the
  * rfunctions are small (at most 10 cells an operation at the widest locus, 16
- * with more tasks than warps fit the GPU);
- * else it times 32, 16, 8 and (in FP64, or with that many tasks) 4 lanes before the first L-sampler work and
- * keeps the fastest, sharing the choice between contexts of one pedigree size
- * class.  These four force one (all forms draw the same graphs).  GENERIC4 fails
+ * with more tasks than warps fit the GPU); else it times 32, 16, 8 and (in FP64,
+ * or with that many tasks) 4 lanes before the first L-sampler work, those whose
+ * arenas fit a block, and keeps the fastest, sharing the choice between contexts
+ * of one pedigree size class.  These four force one (all forms draw the same graphs).  GENERIC4 fails
  * sl_create for a peel sequence outside its limits: cutsets of at most 8
  * members, 16 children per parent peel, every cutset member peeled by a later
  * operation. */

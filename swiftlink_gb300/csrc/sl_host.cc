@@ -49,7 +49,7 @@ cudaError_t launch_msampler(const ProblemDev& P, uint32_t* dg, int first, int nc
                             uint8_t* maps, int* status, int fag_threads, int exact, cudaStream_t s,
                             const uint64_t* key = nullptr, double* ubuf = nullptr, int chains = 1, int load = 1);
 int64_t msweep_launches(const ProblemDev& P, int chains, int nm);
-cudaError_t launch_pack(const int32_t* src, int n, int N, int F, int M, int W, uint32_t* dst, cudaStream_t s);
+cudaError_t launch_pack(const int32_t* src, int n, int N, int F, int M, int W, uint32_t* dst, int sms, cudaStream_t s);
 cudaError_t launch_set_key(uint64_t* key, uint64_t seed, uint64_t iter, cudaStream_t s);
 cudaError_t launch_lfreq(const double* minor, float2* out, int64_t n, cudaStream_t s);
 cudaError_t launch_si(const ProblemDev& P, uint32_t* dg, int first, int nchain, const int32_t* starts,
@@ -2161,9 +2161,13 @@ static int stage_host(sl_ctx* ctx, size_t words) {
 }
 
 // Whether the device takes the caller's graphs from the caller's memory
-// itself: from 256 KB of them on; below, the host's copy is as quick.  (Not the
-// other way: 256 MB unpacked into touched pages took as long as by the host's
-// cores, 2.6 ms, and into new pages four times as long.)
+// itself: from 256 KB of them on.  A scoring call of 30 members, by the host's copy
+// | by the device: 281 KB 95 | 64 us, 750 KB 174 | 102.  Below, a call is short
+// either way and the host's copy keeps it clear of a cold page's cost to the
+// device (touch_pages), though with pages in use the device is the quicker there
+// too: 234 KB 88 | 61, 46 KB 55 | 46.  (Not the other way: 256 MB unpacked into
+// touched pages took as long as by the host's cores, 2.6 ms, and into new pages
+// four times as long.)
 static bool through_pages(const sl_ctx* ctx, int n) {
     return ctx->host_pages && (size_t)n * ctx->P.M * ctx->P.N * 8 >= (256u << 10);
 }
@@ -2186,7 +2190,7 @@ static int queue_graphs(sl_ctx* ctx, const int32_t* dgs, int n, uint32_t* dst, s
     const ProblemDev& P = ctx->P;
     if (through_pages(ctx, n)) {
         touch_pages(ctx, dgs, n);
-        CK(launch_pack(dgs, n, P.N, P.F, P.M, P.W, dst, ctx->stream));
+        CK(launch_pack(dgs, n, P.N, P.F, P.M, P.W, dst, ctx->sms, ctx->stream));
         return SL_OK;
     }
     buf.resize((size_t)P.M * P.W * n);
@@ -2226,7 +2230,7 @@ int sl_set_descent_graphs(sl_ctx* ctx, int32_t first, int32_t n, const int32_t* 
     CK(cudaSetDevice(ctx->device));
     if (through_pages(ctx, n)) {
         touch_pages(ctx, dg, n);
-        CK(launch_pack(dg, n, P.N, P.F, P.M, P.W, ctx->d_dg + words * first, ctx->stream));
+        CK(launch_pack(dg, n, P.N, P.F, P.M, P.W, ctx->d_dg + words * first, ctx->sms, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         return SL_OK;
     }

@@ -2749,11 +2749,11 @@ size_t ffbs_scan_smem(int M) { return ffbs_scan_scratch(ffbs_scan_threads(M)) + 
 // be, evaluates it itself (one step in two to four of the whole cluster).
 //
 // Measured, a sweep of every chain, as launches per meiosis, by a cluster, with
-// the steps evaluated together: 400 members, 10,000 SNPs, 8 chains 128 | 24.2 |
-// 23.0 ms (19.8 in clusters of 11 blocks, msw_choose); 120 members, 2,000 SNPs, 10 chains 5.1 | 2.66 | 2.16 ms (11 us a
-// meiosis), one chain 2.08 | 1.86; 30 members, 200 SNPs 0.39 | 0.335.  (400
-// members, 32 chains, in clusters of 4 blocks, whose bulk hid the evaluations
-// already: 35.9 | 37.3.)  Bound by the evaluated likelihoods
+// the steps evaluated together: 400 members, 10,000 SNPs, one chain 39 | 16.6 |
+// 13.3 ms, 8 chains 128 | 20.8 | 17.8, 32 chains 397 | 37.4 | 35.5; 120 members,
+// 2,000 SNPs, one chain 3.3 | 2.22 | 1.86, 10 chains 5.1 | 2.77 | 2.20 (11 us a
+// meiosis), 160 chains 53 | 8.9 | 8.6; 30 members, 200 SNPs 0.41 | 0.33 (by a
+// cluster).  Bound by the evaluated likelihoods
 // (issue with 32 warps on an SM: 23,000 of a 400-member step's 60,000 cycles;
 // 4,800 of 25,000 for 120 members), by waiting for the block with the most of
 // them (13,000; 5,600) and by the scans' serial runs and barriers.
@@ -2789,9 +2789,10 @@ constexpr size_t kMswSmem = 200 * 1024;
 
 // The shape with up to `cs` blocks per cluster; false when a block's share
 // does not fit its shared memory.  A block has a warp for every four of its
-// loci, where one in 14 is evaluated at a step: with 16 warps for 64 loci (30
-// members, 200 markers) a sweep took 0.40 ms, with 32 0.41; with 32 warps for
-// 640 loci (400 members) 20.4 ms, with 16 26.3.
+// loci, up to 32: of 8, 16 and 32 warps the most are the fastest or as fast.  A
+// sweep with 8 | 16 | 32: 30 members, 200 SNPs 0.354 | 0.328 | 0.329 ms; 120 members,
+// 2,000 SNPs, one chain 2.27 | 1.92 | 1.86, 160 chains 8.6 with any; 400 members, 10,000
+// SNPs, one chain 26.0 | 17.2 | 13.3, 32 chains 59.9 | 36.2 | 35.5.
 static bool msw_shape(const ProblemDev& P, int G, int eb, int cs, MswShape* out) {
     MswShape s;
     s.nw = ffbs_scan_threads(P.M) / 32;
@@ -4789,9 +4790,9 @@ __global__ void __launch_bounds__(256) pack_kernel(const int32_t* __restrict__ s
     }
 }
 
-cudaError_t launch_pack(const int32_t* src, int n, int N, int F, int M, int W, uint32_t* dst, cudaStream_t s) {
+cudaError_t launch_pack(const int32_t* src, int n, int N, int F, int M, int W, uint32_t* dst, int sms, cudaStream_t s) {
     const int64_t words = (int64_t)n * M * W, need = (words + 8 * kPackWords - 1) / (8 * kPackWords);
-    pack_kernel<<<(int)std::min<int64_t>(need, 1216), 256, 0, s>>>(src, N, F, W, words, dst);
+    pack_kernel<<<(int)std::min<int64_t>(need, 8 * (int64_t)sms), 256, 0, s>>>(src, N, F, W, words, dst);
     return cudaGetLastError();
 }
 // log2 of each chain's major and minor allele frequency at each locus, in
