@@ -3118,6 +3118,7 @@ int sl_trait_backward(sl_ctx* ctx, int32_t n_graphs, const int32_t* dgs, double*
         return SL_OK;
     };
     if (n_graphs == 0) {
+        if (!ptrait_grad) return SL_OK;   // nothing asked for: what is queued, and its status, stay as they are
         if ((rc = sl_synchronize(ctx))) return rc;
         return ptrait();
     }
